@@ -184,31 +184,33 @@ def _fill_cache(ctx, views, rows, gen, rng):
 
 
 def _set_norms(ctx, case, gen):
-    if not case.get("norm"):
-        return
-    for layer in range(case["layers"]):
+    """QK-norm weights per layer, or an empty list."""
+    norms = []
+    for layer in range(case["layers"] if case.get("norm") else 0):
         qn, kn = (1.0 + 0.2 * torch.randn(2, ctx.config.head_dim, generator=gen, device="cuda")).cpu().numpy()
         ctx.set_layer_fixups(layer, q_norm=qn, k_norm=kn, eps=1e-6)
+        norms.append((qn, kn))
+    return norms
 
 
 def _weights(kind, rows, cols, rng):
-    """A projection matrix of N(0, 0.02)-like weights in the row layout of the model file."""
+    """A projection matrix of N(0, 0.02)-like weights in the row layout of the model file: (type, rows, cols, data)."""
     n = rows * cols
     if kind in ("f32", "bf16"):
         w = (rng.standard_normal((rows, cols), dtype=np.float32) * 0.02)
-        return Weights(W_F32, rows, cols, w) if kind == "f32" else Weights(W_BF16, rows, cols, (w.view(np.uint32) >> 16).astype(np.uint16))
+        return (W_F32, rows, cols, w) if kind == "f32" else (W_BF16, rows, cols, (w.view(np.uint32) >> 16).astype(np.uint16))
     if kind == "q8_0":
         blocks = np.frombuffer(rng.bytes(n // 32 * 34), np.uint8).reshape(-1, 34).copy()
         blocks[:, :2] = (rng.uniform(0.8, 1.2, n // 32) * 0.02 / 74).astype(np.float16).view(np.uint8).reshape(-1, 2)
-        return Weights(W_Q8_0, rows, cols, blocks)
+        return W_Q8_0, rows, cols, blocks
     if kind == "q4_k":
         blocks = np.frombuffer(rng.bytes(n // 256 * 144), np.uint8).reshape(-1, 144).copy()
         d = rng.uniform(0.8, 1.2, (n // 256, 2)) * np.array([1.0, 7.5]) * 0.02 / 250
         blocks[:, :4] = d.astype(np.float16).view(np.uint8).reshape(-1, 4)
-        return Weights(W_Q4_K, rows, cols, blocks)
+        return W_Q4_K, rows, cols, blocks
     blocks = np.frombuffer(rng.bytes(n // 256 * 210), np.uint8).reshape(-1, 210).copy()
     blocks[:, 208:] = (rng.uniform(0.8, 1.2, n // 256) * 0.02 / 1360).astype(np.float16).view(np.uint8).reshape(-1, 2)
-    return Weights(W_Q6_K, rows, cols, blocks)
+    return W_Q6_K, rows, cols, blocks
 
 
 def _layer_weights(case, layer, rng):
@@ -231,14 +233,14 @@ def prepare(case, seed):
     ctx = g.AttnContext(_config(case, case["ctx"] if decode else case["base"] + case["m"]))
     views = _cache_views(ctx)
     _fill_cache(ctx, views, first, gen, rng)
-    _set_norms(ctx, case, gen)
-    state = {"case": case, "ctx": ctx, "layers": range(layers)}
+    norms = _set_norms(ctx, case, gen)
+    state = {"case": case, "ctx": ctx, "layers": range(layers), "views": views, "norms": norms}
 
     def randn(*shape):
         return torch.randn(*shape, generator=gen, device="cuda")
 
     if case["kind"] in ("layer_decode", "layer_prefill"):
-        state["w"] = [_layer_weights(case, layer, rng) for layer in range(layers)]
+        state["w"] = [[Weights(*w) for w in _layer_weights(case, layer, rng)] for layer in range(layers)]
         state["x"] = list(randn(layers, rows, hidden))
         out = torch.empty(layers, rows, hidden, device="cuda")
     else:
@@ -321,3 +323,121 @@ def tolerance(case):
     if case["kv"] == "bf16" or (case["kv"] == "turbo" and case["kind"] == "decode"):
         return {"rel": 1e-2, "differ": 5e-3}
     return {"rel": 1e-5, "differ": 5e-3}
+
+
+def _dense(w):
+    """A projection matrix in 64 bits from its model-file bytes (the GGML block layouts)."""
+    wtype, rows, cols, data = w
+    if wtype in (W_F32, W_BF16):
+        d = data if wtype == W_F32 else (data.astype(np.uint32) << 16).view(np.float32)
+        return torch.from_numpy(d).cuda().double()
+    b = torch.from_numpy(data).cuda()
+
+    def halves(cols_):
+        return b[:, cols_].contiguous().view(torch.float16).double()
+
+    if wtype == W_Q8_0:
+        out = halves(slice(0, 2)) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif wtype == W_Q4_K:  # d, dmin, twelve bytes of eight 6-bit (scale, min) pairs, nibbles in groups of 64
+        sc, qs = b[:, 4:16].int(), b[:, 16:].reshape(-1, 4, 32)
+        scale = torch.cat([sc[:, :4] & 63, (sc[:, 8:] & 15) | (sc[:, :4] >> 6 << 4)], 1)
+        low = torch.cat([sc[:, 4:8] & 63, (sc[:, 8:] >> 4) | (sc[:, 4:8] >> 6 << 4)], 1)
+        q = torch.stack([qs & 15, qs >> 4], 2).reshape(-1, 8, 32).double()
+        out = (halves(slice(0, 2)) * scale)[..., None] * q - (halves(slice(2, 4)) * low)[..., None]
+    else:  # Q6_K: low nibbles, high bit pairs, sixteen int8 scales, d
+        lo, hi = b[:, :128].reshape(-1, 2, 64).int(), b[:, 128:192].reshape(-1, 2, 32).int()
+        q = torch.stack([(lo[..., :32] & 15) | (hi & 3) << 4, (lo[..., 32:] & 15) | (hi >> 2 & 3) << 4,
+                         (lo[..., :32] >> 4) | (hi >> 4 & 3) << 4, (lo[..., 32:] >> 4) | (hi >> 6 & 3) << 4], 2)
+        scale = halves(slice(208, 210)) * b[:, 192:208].contiguous().view(torch.int8).double()
+        out = scale[..., None] * (q.reshape(-1, 16, 16) - 32).double()
+    return out.reshape(rows, cols)
+
+
+def _rotate(x, pos, theta, style):
+    """RoPE of x [rows][heads][dim] in 64 bits; frequencies and angles are f32, as the models define them."""
+    dim = x.shape[-1]
+    power = (float(theta) ** (np.arange(0, dim, 2, dtype=np.float32) / np.float32(dim)).astype(np.float64)).astype(np.float32)
+    freq = np.float32(1.0) / power
+    angle = torch.from_numpy(np.asarray(pos, np.float32)[:, None] * freq).cuda().double()[:, None]
+    c, s = angle.cos(), angle.sin()
+    a, b = (x[..., :dim // 2], x[..., dim // 2:]) if style == ROPE_NEOX else (x[..., ::2], x[..., 1::2])
+    pair = a * c - b * s, a * s + b * c
+    return torch.cat(pair, -1) if style == ROPE_NEOX else torch.stack(pair, -1).flatten(-2)
+
+
+def _stored(x, kv):
+    """Rows [n][elements] as the cache holds them: values in 64 bits, and the scales of a q8 cache."""
+    if kv in ("f32", "bf16"):
+        return (x.float().double() if kv == "f32" else x.float().bfloat16().double()), None
+    blocks = x.float().reshape(x.shape[0], -1, 32 if kv == "q8_block32" else x.shape[1])
+    top = blocks.abs().amax(-1, keepdim=True)
+    codes = (blocks * (127.0 / top)).double()
+    codes = torch.sign(codes) * torch.floor(codes.abs() + 0.5)
+    return (codes * (top / 127.0)).reshape(x.shape), (top / 127.0)[..., 0]
+
+
+def _attend(q, k, v, ends, window):
+    """q [rows][heads][dim] over k, v [keys][kv_heads][dim]; row i sees keys max(0, ends[i] - window) .. ends[i] - 1."""
+    group, at = q.shape[1] // k.shape[1], torch.arange(k.shape[0], device="cuda")
+    out = torch.empty_like(q)
+    hide = (at >= ends[:, None]) | (at < ends[:, None] - window if window else torch.zeros_like(at, dtype=torch.bool))
+    for h in range(q.shape[1]):
+        s = (q[:, h] @ k[:, h // group].T) * q.shape[-1] ** -0.5
+        out[:, h] = torch.softmax(s.masked_fill_(hide, -torch.inf), -1) @ v[:, h // group]
+    return out
+
+
+def exact(case, seed):
+    """What a pass leaves, in 64 bits from the stored cache rows. Codes of quantised caches have no such value, and the
+    TurboQuant cache none that is not made of the same transforms."""
+    if case["kv"] == "turbo":
+        return None
+    heads, kv_heads, dim, _, style, theta, _ = SHAPES[case["shape"]]
+    state = prepare(case, seed)
+    views, layers = state["views"], case["layers"]
+    decode = case["kind"] in ("decode", "layer_decode")
+    pos = state["pos"] if decode else np.arange(case["base"], case["base"] + case["m"])
+    windows = (gemma_layer_windows(layers, GEMMA_WINDOW, 6) if case["shape"] == "gemma3_4b" else [0] * layers)
+    rng, outs, rows_k, rows_v, scales = np.random.default_rng(seed), [], [], [], []
+    for layer in range(layers):
+        if "weights" in case:
+            w = [_dense(x) for x in _layer_weights(case, layer, rng)]
+            q, k, v = (state["x"][layer].double() @ m.T for m in w[:3])
+        else:
+            q, k, v = (torch.as_tensor(state[n][layer]).cuda().double() for n in "qkv")
+        n = q.shape[0]
+        q, k = q.reshape(n, heads, dim), k.reshape(n, kv_heads, dim)
+        if state["norms"]:
+            q, k = (x * (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * torch.from_numpy(g_).cuda().double()
+                    for x, g_ in zip((q, k), state["norms"][layer]))
+        th = 1e4 if windows[layer] else theta
+        q, k = _rotate(q, pos, th, style), _rotate(k, pos, th, style).reshape(n, -1)
+        (k_kept, k_scale), (v_kept, v_scale) = _stored(k, case["kv"]), _stored(v, case["kv"])
+        rows_k.append(k)
+        rows_v.append(v)
+        scales.append((k_scale, v_scale))
+        out = torch.empty_like(q)
+        for b in range(n if decode else 1):
+            first = int(pos[b]) if decode else case["base"]
+            old = [a[b, layer, :first].double() for a in views[:2]]
+            for i, s in enumerate(views[2:]):
+                s = s[b, layer, :first].double()
+                old[i] = (old[i].reshape(first, s.shape[1], old[i].shape[1] // s.shape[1]) * s[..., None]).flatten(1)
+            sel = slice(b, b + 1) if decode else slice(None)
+            kk, vv = (torch.cat([o, r[sel]]).reshape(-1, kv_heads, dim) for o, r in zip(old, (k_kept, v_kept)))
+            out[sel] = _attend(q[sel], kk, vv, torch.as_tensor(pos[sel], device="cuda") + 1, windows[layer])
+        out = out.reshape(n, -1)
+        outs.append(out @ w[3].T if "weights" in case else out)
+
+    def as_appended(rows):  # [sequence][layer][position][...]
+        x = torch.stack(rows)
+        return x.transpose(0, 1)[:, :, None] if decode else x[None]
+
+    if decode and case["ragged"]:
+        coded = case["kv"].startswith("q8")
+        appended = [None if coded else as_appended(rows_k)[b, :, 0] for b in range(min(16, case["batch"]))]
+    elif scales[0][0] is not None:
+        appended = [None, None, as_appended([s[0] for s in scales]), as_appended([s[1] for s in scales])]
+    else:
+        appended = [as_appended(rows_k), as_appended(rows_v)]
+    return {"out": torch.stack(outs), "appended": appended}
