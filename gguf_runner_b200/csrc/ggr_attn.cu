@@ -19,6 +19,7 @@
 #include "attn_turbo.cuh"
 #include "attn_turbo_mma.cuh"
 #include "common.cuh"
+#include "prefill_split.cuh"
 #include "prefill_tc.cuh"
 #include "prefill_tc_wide.cuh"
 #include "proj.cuh"
@@ -767,6 +768,49 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     return launch_simt(c, a, grid, p);
 }
 
+// Prefill rows of a quantised cache on the tensor cores in 32-bit precision (prefill_split.cuh); `q_dev` holds rotated
+// queries, the rows are appended already.
+int launch_split_prefill(ggr_attn_ctx* c, int layer, const Items& items, int t_max, const float* q_dev, float* out_dev,
+                         const GateSpec& gate) {
+    AttnArgs a{};
+    a.kv = c->kv;
+    a.items = items;
+    a.vis = visibility(c, layer);
+    a.layer = layer;
+    a.q = q_dev;
+    a.score_scale = (c->cfg.scale_mode == GGR_SCALE_SCORE ? c->attn_scale : 1.0f) * kLog2e;
+    a.out = out_dev;
+    a.shard_count = c->shard_count;
+    if (gate.p) {
+        a.gate = static_cast<const float*>(gate.p);
+        a.gate_head_stride = gate.head_stride;
+    }
+    const int row_tiles = (items.n * c->G + kPsRows - 1) / kPsRows;
+    const int slots = c->sm_count * (c->kv.fmt == KV_TURBO ? 1 : 2);
+    int limit = std::min(kPsMaxSplits, (t_max + 255) / 256);
+    if (c->cfg.max_splits > 0) limit = std::min(limit, c->cfg.max_splits);
+    const int n_split = std::max(1, std::min(limit, slots / (row_tiles * c->kv.Hkv)));
+    a.n_split = n_split;
+    c->last_splits = n_split;
+    if (n_split > 1) {
+        int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)items.n * c->kv.Hq * n_split * (c->D + 2));
+        if (rc) return rc;
+        const size_t before = c->counters_cap;
+        rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)row_tiles * c->kv.Hkv);
+        if (rc) return rc;
+        if (c->counters_cap != before)
+            CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, c->counters_cap * sizeof(unsigned), c->stream));
+        a.part = c->d_part;
+        a.counters = c->d_counters;
+    }
+    {
+        LaunchTimer t(c, 0);
+        CUDA_TRY(c, launch_prefill_split(a, dim3(c->kv.Hkv, row_tiles, n_split), c->smem_optin, c->cfg.device, c->stream));
+    }
+    c->launches++;
+    return GGR_OK;
+}
+
 // copies a caller buffer into a staging slot when the caller's memory is host memory
 int stage_in(ggr_attn_ctx* c, int slot, const void* src, size_t bytes, int ptr_kind, const void** dev) {
     if (ptr_kind == GGR_PTR_DEVICE) {
@@ -1090,8 +1134,11 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
                     gs.p = reinterpret_cast<const float*>(dgate) + (size_t)j0 * gate_row;
                 }
             }
-            int r = launch_attention(c, layer, it, t_max, c->d_qrot + (size_t)j0 * c->q_dim, dout + (size_t)j0 * c->q_dim,
-                                     nullptr, false, nullptr, nullptr, &gs);
+            const float* qr = c->d_qrot + (size_t)j0 * c->q_dim;
+            float* o = dout + (size_t)j0 * c->q_dim;
+            int r = c->cfg.prefill_impl == GGR_IMPL_AUTO && prefill_split_supported(c->kv.fmt, c->D)
+                        ? launch_split_prefill(c, layer, it, t_max, qr, o, gs)
+                        : launch_attention(c, layer, it, t_max, qr, o, nullptr, false, nullptr, nullptr, &gs);
             if (r) return r;
         }
         return GGR_OK;
