@@ -171,4 +171,28 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+// Kernels of the library that follow one another on a stream are launched programmatically behind each other
+// (launch_chained): the next grid's CTAs take the slots that drain while the last CTAs of the one before it finish, so
+// the launch, the CTA start-up and what does not depend on the predecessor (barriers, tensor memory, weights) cost no
+// time of their own. Every kernel launched that way calls grid_wait() before it touches memory that any earlier work
+// in the stream may write or read; that covers work of other origin too, since the predecessor has waited likewise.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream,
+                                  A&&... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(block);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace ggr

@@ -235,6 +235,18 @@ void visible_host(const ggr_attn_ctx* c, int layer, int pos, int* vs, int* ve) {
     *ve = e;
 }
 
+// Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, and not
+// into a stream capture, where the node in front may be a copy or an event of the caller's.
+bool chain_launches(const ggr_attn_ctx* c) {
+    if (c->timing) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
 // Brackets one launch with events when kernel timing is on.
 struct LaunchTimer {
     ggr_attn_ctx* c;
@@ -2270,7 +2282,7 @@ struct ggr_weights {
     __half2* d_dm = nullptr;           // Q4_K: (d, dmin) per super-block [rows][cols / 256]
     float* d_scales_f32 = nullptr;     // Q6_K: d * scale per 16 weights [rows][cols / 16]
     __nv_bfloat16* d_bf16 = nullptr;   // bf16 image for the tensor-core kernel (d_main itself for BF16)
-    CUtensorMap tmB;                   // [rows][cols] bf16, box 64 x 256
+    CUtensorMap tmB;                   // [rows][cols] bf16, box 64 x 128
     bool have_tmap = false;
 };
 
@@ -2325,6 +2337,52 @@ void fill_gemv(GemvArgs& a, const ggr_weights* w, const float* x, int n, float* 
     a.sanitize = sanitize;
 }
 
+// Output of one matrix of a gemm_device call: f32 or bf16 rows.
+struct GemmOut {
+    const ggr_weights* w;
+    float* out;
+    __nv_bfloat16* out_h;
+    int ld_out;
+};
+
+// x [n][cols] times one to three matrices of the same column count on the tensor cores: one conversion of the rows to
+// bf16, one launch over the column tiles of all of them
+int gemm_device(ggr_attn_ctx* c, const GemmOut* mats, int n_mats, const float* x, int n, int sanitize) {
+    const ggr_weights* w = mats[0].w;
+    const CUtensorMap* maps[3] = {};
+    GemmArgs g{};
+    for (int i = 0; i < n_mats; ++i) {
+        if (mats[i].w->device != c->cfg.device) return fail(c, GGR_ERR_INVALID, "the weights live on another device than the context");
+        if (!mats[i].w->have_tmap) return fail(c, GGR_ERR_UNSUPPORTED, "no tensor map for these weights (driver entry point missing)");
+        maps[i] = &mats[i].w->tmB;
+        g.N[i] = mats[i].w->rows;
+        g.out[i] = mats[i].out;
+        g.out_h[i] = mats[i].out_h;
+        g.ld_out[i] = mats[i].ld_out;
+    }
+    int rc = ensure(c, &c->d_pact, &c->pact_cap, (size_t)n * w->cols);
+    if (rc) return rc;
+    const bool chained = chain_launches(c);
+    const size_t elems = (size_t)n * w->cols;
+    CUDA_TRY(c, launch_chained(chained, proj_to_bf16_kernel, dim3((unsigned)std::min<size_t>(2048, (elems / 4 + 255) / 256 + 1)), 256,
+                               0, c->stream, x, c->d_pact, elems));
+    c->launches++;
+    CUtensorMap tmA;
+    if (!make_tmap_bf16(&tmA, c->d_pact, (uint64_t)w->cols, (uint64_t)n, kGemmBM))
+        return fail(c, GGR_ERR_CUDA, "cuTensorMapEncodeTiled failed for the activation rows");
+    g.m = n;
+    g.K = w->cols;
+    g.n_mats = n_mats;
+    g.sanitize = sanitize;
+    g.err = c->d_err;
+    {
+        LaunchTimer t(c, 3);
+        CUDA_TRY(c, launch_gemm(tmA, maps, g, chained, c->cfg.device, c->sm_count, c->stream));
+    }
+    c->launches++;
+    return GGR_OK;
+}
+
 int matmul_device(ggr_attn_ctx* c, const ggr_weights* w, const float* x, int n, float* out, __nv_bfloat16* out_h, int ld_out,
                   int sanitize) {
     if (w->device != c->cfg.device) return fail(c, GGR_ERR_INVALID, "the weights live on another device than the context");
@@ -2338,31 +2396,21 @@ int matmul_device(ggr_attn_ctx* c, const ggr_weights* w, const float* x, int n, 
         c->launches++;
         return GGR_OK;
     }
-    if (!w->have_tmap) return fail(c, GGR_ERR_UNSUPPORTED, "no tensor map for these weights (driver entry point missing)");
-    int rc = ensure(c, &c->d_pact, &c->pact_cap, (size_t)n * w->cols);
-    if (rc) return rc;
-    const size_t elems = (size_t)n * w->cols;
-    proj_to_bf16_kernel<<<(unsigned)std::min<size_t>(2048, (elems / 4 + 255) / 256 + 1), 256, 0, c->stream>>>(x, c->d_pact, elems);
-    CUDA_TRY(c, cudaGetLastError());
-    c->launches++;
-    CUtensorMap tmA;
-    if (!make_tmap_bf16(&tmA, c->d_pact, (uint64_t)w->cols, (uint64_t)n, kGemmBM))
-        return fail(c, GGR_ERR_CUDA, "cuTensorMapEncodeTiled failed for the activation rows");
-    GemmArgs g{};
-    g.m = n;
-    g.N = w->rows;
-    g.K = w->cols;
-    g.out = out;
-    g.out_h = out_h;
-    g.ld_out = ld_out;
-    g.sanitize = sanitize;
-    g.err = c->d_err;
-    {
-        LaunchTimer t(c, 3);
-        CUDA_TRY(c, launch_gemm(tmA, w->tmB, g, c->cfg.device, c->stream));
+    const GemmOut mat{w, out, out_h, ld_out};
+    return gemm_device(c, &mat, 1, x, n, sanitize);
+}
+
+// the q, k and v projections of the same rows
+int matmul_qkv_device(ggr_attn_ctx* c, const ggr_weights* wq, const ggr_weights* wk, const ggr_weights* wv, const float* x, int n,
+                      float* q, float* k, float* v) {
+    if (n > 16 || wq->cols > kGemvMaxCols) {
+        const GemmOut mats[3] = {{wq, q, nullptr, c->q_dim}, {wk, k, nullptr, c->kv_dim}, {wv, v, nullptr, c->kv_dim}};
+        return gemm_device(c, mats, 3, x, n, 0);
     }
-    c->launches++;
-    return GGR_OK;
+    int rc;
+    if ((rc = matmul_device(c, wq, x, n, q, nullptr, c->q_dim, 0))) return rc;
+    if ((rc = matmul_device(c, wk, x, n, k, nullptr, c->kv_dim, 0))) return rc;
+    return matmul_device(c, wv, x, n, v, nullptr, c->kv_dim, 0);
 }
 
 int check_layer_weights(ggr_attn_ctx* c, const ggr_weights* wq, const ggr_weights* wk, const ggr_weights* wv,
@@ -2517,7 +2565,7 @@ extern "C" int ggr_weights_upload(int32_t device, int32_t wtype, int32_t rows, i
         if (cudaMalloc((void**)&w->d_bf16, n * 2) != cudaSuccess) return fail_up("unable to allocate the bf16 weight image");
         if (cudaMemcpy(w->d_bf16, image.data(), n * 2, cudaMemcpyHostToDevice) != cudaSuccess) return fail_up("weight upload failed");
     }
-    w->have_tmap = make_tmap_bf16(&w->tmB, w->d_bf16, (uint64_t)cols, (uint64_t)rows, kGemmBN);
+    w->have_tmap = make_tmap_bf16(&w->tmB, w->d_bf16, (uint64_t)cols, (uint64_t)rows, kGemmBoxN);
     g_create_err.clear();
     *out = w;
     return GGR_OK;
@@ -2610,9 +2658,7 @@ extern "C" int ggr_attn_layer_decode(ggr_attn_ctx* c, int32_t layer, const int32
         }
         c->launches++;
     } else {
-        if ((rc = matmul_device(c, wq, dx, B, dq, nullptr, c->q_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wk, dx, B, dk, nullptr, c->kv_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wv, dx, B, dv, nullptr, c->kv_dim, 0))) return rc;
+        if ((rc = matmul_qkv_device(c, wq, wk, wv, dx, B, dq, dk, dv))) return rc;
     }
     if ((rc = decode_common(c, layer, pos, B, dq, dk, dv, c->d_patt, nullptr, GGR_PTR_DEVICE))) return rc;
     if ((rc = matmul_device(c, wo, c->d_patt, B, dout, nullptr, dim_out, 1))) return rc;
@@ -2657,18 +2703,15 @@ extern "C" int ggr_attn_layer_prefill(ggr_attn_ctx* c, int32_t layer, int32_t se
         __nv_bfloat16* hq = c->d_pqkv_h;
         __nv_bfloat16* hk = hq + (size_t)m * c->q_dim;
         __nv_bfloat16* hv = hk + (size_t)m * c->kv_dim;
-        if ((rc = matmul_device(c, wq, dx, m, nullptr, hq, c->q_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wk, dx, m, nullptr, hk, c->kv_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wv, dx, m, nullptr, hv, c->kv_dim, 0))) return rc;
+        const GemmOut mats[3] = {{wq, nullptr, hq, c->q_dim}, {wk, nullptr, hk, c->kv_dim}, {wv, nullptr, hv, c->kv_dim}};
+        if ((rc = gemm_device(c, mats, 3, dx, m, 0))) return rc;
         rc = prefill_common(c, layer, seq, base_pos, m, hq, hk, hv, GGR_DTYPE_BF16, c->d_patt, GGR_PTR_DEVICE, false);
     } else {
         if ((rc = ensure(c, &c->d_pqkv, &c->pqkv_cap, (size_t)m * qkv))) return rc;
         float* dq = c->d_pqkv;
         float* dk = dq + (size_t)m * c->q_dim;
         float* dv = dk + (size_t)m * c->kv_dim;
-        if ((rc = matmul_device(c, wq, dx, m, dq, nullptr, c->q_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wk, dx, m, dk, nullptr, c->kv_dim, 0))) return rc;
-        if ((rc = matmul_device(c, wv, dx, m, dv, nullptr, c->kv_dim, 0))) return rc;
+        if ((rc = matmul_qkv_device(c, wq, wk, wv, dx, m, dq, dk, dv))) return rc;
         rc = prefill_common(c, layer, seq, base_pos, m, dq, dk, dv, GGR_DTYPE_F32, c->d_patt, GGR_PTR_DEVICE, false);
     }
     if (rc) return rc;

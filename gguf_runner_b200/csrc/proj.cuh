@@ -12,8 +12,8 @@
 //                     d * scale * sum(x q) - dmin * min * sum(x), one FMA per weight) and Q6_K (kept as int8 codes
 //                     q - 32 with one f32 scale per 16 weights, which is one lane's load).
 //   proj_gemm_kernel  prefill chunks: tcgen05 GEMM, bf16 x bf16 -> f32 in TMEM. A = activations [m][K] (bf16), B =
-//                     weights [N][K] (bf16; Q8_0 / F32 weights use a bf16 image made at upload), 128 x 256 output
-//                     tile per CTA, 64-column k-steps through a four-stage TMA ring, one MMA issuer, four epilogue
+//                     weights [N][K] (bf16; Q8_0 / F32 weights use a bf16 image made at upload), 128 x 256 or
+//                     128 x 128 output tile per CTA, 64-column k-steps through a four- or six-stage TMA ring, one MMA issuer, four epilogue
 //                     warps reading the accumulator out of TMEM. Every wait is bounded.
 #pragma once
 
@@ -374,6 +374,8 @@ inline cudaError_t launch_gemv(int wtype, const GemvArgs& a, int device, int sm_
 
 // f32 rows -> bf16 rows (activations on their way into the tensor-core GEMM)
 __global__ void proj_to_bf16_kernel(const float* src, __nv_bfloat16* dst, size_t n) {
+    grid_allow_dependents();
+    grid_wait();
     for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (size_t)gridDim.x * blockDim.x * 4) {
         if (i + 4 <= n) {
             const float4 v = *reinterpret_cast<const float4*>(src + i);
@@ -390,39 +392,54 @@ __global__ void proj_to_bf16_kernel(const float* src, __nv_bfloat16* dst, size_t
 
 // ---- tcgen05 GEMM ------------------------------------------------------------------------------------------
 
+// Up to three matrices of one column count (the q, k and v projections) multiplied with the same rows in one launch:
+// their column tiles are numbered one after the other.
 struct GemmArgs {
-    int m, N, K;
-    float* out;             // [m][ld_out] f32, or null
-    __nv_bfloat16* out_h;   // [m][ld_out] bf16, or null
-    int ld_out;
+    int m, K;
+    int n_mats;
+    int N[3];
+    int tile0[3];              // first column tile of each matrix
+    float* out[3];             // [m][ld_out] f32, or null
+    __nv_bfloat16* out_h[3];   // [m][ld_out] bf16, or null
+    int ld_out[3];
     int sanitize;
     int* err;               // raised when a bounded wait runs out
 };
 
-constexpr int kGemmBM = 128, kGemmBN = 256, kGemmBK = 64, kGemmStages = 4;
+constexpr int kGemmBM = 128, kGemmBK = 64;
+constexpr int kGemmBoxN = 128;     // weight rows of one TMA box
 constexpr int kGemmThreads = 192;  // four epilogue warps, a TMA producer, an MMA issuer
-constexpr uint32_t kGemmABytes = kGemmBM * kGemmBK * 2, kGemmBBytes = kGemmBN * kGemmBK * 2;
-inline size_t proj_gemm_smem() { return (size_t)kGemmStages * (kGemmABytes + kGemmBBytes) + 1024; }
+constexpr uint32_t kGemmABytes = kGemmBM * kGemmBK * 2, kGemmBoxBytes = kGemmBoxN * kGemmBK * 2;
+template <int BN>
+struct GemmGeom {
+    static constexpr int STAGES = BN == 256 ? 4 : 6;  // 192 KB either way
+    static constexpr uint32_t BBYTES = BN * kGemmBK * 2;
+    static constexpr size_t SMEM = (size_t)STAGES * (kGemmABytes + BBYTES) + 1024;
+};
 
+template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs a) {
+proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
+                 const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2, GemmArgs a) {
     using namespace tc;
+    constexpr int STAGES = GemmGeom<BN>::STAGES;
+    constexpr uint32_t BBYTES = GemmGeom<BN>::BBYTES;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * kGemmStages + 1];
+    __shared__ __align__(8) uint64_t bars[2 * STAGES + 1];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t sA = smem_base, sB = smem_base + kGemmStages * kGemmABytes;
+    const uint32_t sA = smem_base, sB = smem_base + STAGES * kGemmABytes;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * s; };
-    auto empty = [&](int s) { return bar0 + 8u * (kGemmStages + s); };
-    const uint32_t acc_full = bar0 + 8u * (2 * kGemmStages);
+    auto empty = [&](int s) { return bar0 + 8u * (STAGES + s); };
+    const uint32_t acc_full = bar0 + 8u * (2 * STAGES);
 
     if (tid == 0) {
         s_abort = 0;
-        for (int s = 0; s < kGemmStages; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
         }
@@ -430,37 +447,56 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) {
-        tmem_alloc(smem_u32(&s_tmem_base), kGemmBN);
+        tmem_alloc(smem_u32(&s_tmem_base), BN);
         tmem_relinquish();
     }
+    grid_allow_dependents();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = s_tmem_base;
     volatile int* abortp = &s_abort;
-    const int n0 = blockIdx.x * kGemmBN, m0 = blockIdx.y * kGemmBM;
+    // (selects, not indexed parameter loads)
+    const int bx = blockIdx.x;
+    const int mat = a.n_mats > 2 && bx >= a.tile0[2] ? 2 : (a.n_mats > 1 && bx >= a.tile0[1] ? 1 : 0);
+    const int N = mat == 2 ? a.N[2] : mat == 1 ? a.N[1] : a.N[0];
+    const int ld_out = mat == 2 ? a.ld_out[2] : mat == 1 ? a.ld_out[1] : a.ld_out[0];
+    const int n0 = (bx - (mat == 2 ? a.tile0[2] : mat == 1 ? a.tile0[1] : 0)) * BN, m0 = blockIdx.y * kGemmBM;
     const int nk = (a.K + kGemmBK - 1) / kGemmBK;
 
     if (warp == 4) {
         if (lane == 0) {
+            const CUtensorMap* tmB = mat == 2 ? &tmB2 : mat == 1 ? &tmB1 : &tmB0;
+            auto load_b = [&](int k) {
+                const int s = k % STAGES;
+                mbar_expect_tx(full(s), kGemmABytes + BBYTES);
+#pragma unroll
+                for (int j = 0; j < BN / kGemmBoxN; ++j)
+                    tma_load_2d(sB + s * BBYTES + j * kGemmBoxBytes, tmB, k * kGemmBK, n0 + j * kGemmBoxN, full(s));
+            };
+            // the weights of the first stages do not depend on the kernel in front, which makes the activations
+            const int ahead = min(nk, STAGES);
+            for (int k = 0; k < ahead; ++k) load_b(k);
+            grid_wait();
             for (int k = 0; k < nk; ++k) {
-                const int s = k % kGemmStages;
-                if (!mbar_wait(empty(s), ((k / kGemmStages) & 1) ^ 1, abortp)) break;
-                mbar_expect_tx(full(s), kGemmABytes + kGemmBBytes);
+                const int s = k % STAGES;
+                if (k >= ahead) {
+                    if (!mbar_wait(empty(s), ((k / STAGES) & 1) ^ 1, abortp)) break;
+                    load_b(k);
+                }
                 tma_load_2d(sA + s * kGemmABytes, &tmA, k * kGemmBK, m0, full(s));
-                tma_load_2d(sB + s * kGemmBBytes, &tmB, k * kGemmBK, n0, full(s));
             }
         }
     } else if (warp == 5) {
-        constexpr uint32_t IDESC = idesc_bf16(kGemmBN, 0);
+        constexpr uint32_t IDESC = idesc_bf16(BN, 0);
         const uint64_t dA = smem_desc(sA, 16, 1024), dB = smem_desc(sB, 16, 1024);
         const uint32_t tm = __shfl_sync(0xffffffffu, s_tmem_base, 0);
         bool ok = true;
         for (int k = 0; k < nk && ok; ++k) {
-            const int s = k % kGemmStages;
-            if (!(ok = mbar_wait_warp(full(s), (k / kGemmStages) & 1, abortp))) break;
+            const int s = k % STAGES;
+            if (!(ok = mbar_wait_warp(full(s), (k / STAGES) & 1, abortp))) break;
             fence_after_sync();
-            const uint64_t a0 = dA + (uint64_t)((s * kGemmABytes) >> 4), b0 = dB + (uint64_t)((s * kGemmBBytes) >> 4);
+            const uint64_t a0 = dA + (uint64_t)((s * kGemmABytes) >> 4), b0 = dB + (uint64_t)((s * BBYTES) >> 4);
 #pragma unroll
             for (int ks = 0; ks < kGemmBK / 16; ++ks)
                 mma_ss_e(tm, a0 + (uint64_t)((ks * 32) >> 4), b0 + (uint64_t)((ks * 32) >> 4), IDESC, (k > 0 || ks > 0) ? 1u : 0u);
@@ -468,21 +504,23 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (ok) mma_commit_e(acc_full);
     } else {
+        float* const out = mat == 2 ? a.out[2] : mat == 1 ? a.out[1] : a.out[0];
+        __nv_bfloat16* const out_h = mat == 2 ? a.out_h[2] : mat == 1 ? a.out_h[1] : a.out_h[0];
         // epilogue: thread = output row of the tile (TMEM lane), 32 columns per tcgen05.ld
         const int row = m0 + warp * 32 + lane;
         if (mbar_wait(acc_full, 0, abortp)) {
             fence_after_sync();
             const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
-            for (int c = 0; c < kGemmBN / 32; ++c) {
+            for (int c = 0; c < BN / 32; ++c) {
                 uint32_t v[32];
                 tmem_ld32(t0 + c * 32, v);
                 tmem_wait_ld();
                 const int col0 = n0 + c * 32;
-                if (row < a.m && col0 < a.N) {
-                    const int ncol = min(32, a.N - col0);
-                    if (a.out) {
-                        float* o = a.out + (size_t)row * a.ld_out + col0;
+                if (row < a.m && col0 < N) {
+                    const int ncol = min(32, N - col0);
+                    if (out) {
+                        float* o = out + (size_t)row * ld_out + col0;
                         for (int i = 0; i < ncol; i += 4) {
                             float4 f = make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
                                                    __uint_as_float(v[i + 3]));
@@ -495,8 +533,8 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                             *reinterpret_cast<float4*>(o + i) = f;
                         }
                     }
-                    if (a.out_h) {
-                        __nv_bfloat16* o = a.out_h + (size_t)row * a.ld_out + col0;
+                    if (out_h) {
+                        __nv_bfloat16* o = out_h + (size_t)row * ld_out + col0;
                         for (int i = 0; i < ncol; i += 2) {
                             __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
                             *reinterpret_cast<__nv_bfloat162*>(o + i) = p;
@@ -512,20 +550,39 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    if (warp == 5) tmem_dealloc(tmem, kGemmBN);
+    if (warp == 5) tmem_dealloc(tmem, BN);
     if (tid == 0 && s_abort && a.err) atomicExch(a.err, 1);
 }
 
-// tmA: activations [m][K] with a 64 x 128 box; tmB: weights [N][K] with a 64 x 256 box
-inline cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, int device,
-                               cudaStream_t stream) {
+// tmA: activations [m][K] with a 64 x 128 box; tmB: weights [N][K] with a 64 x 128 box, one map per matrix
+template <int BN>
+inline cudaError_t launch_gemm_inst(const CUtensorMap& tmA, const CUtensorMap* const* tmB, GemmArgs a, bool chained, int device,
+                                    cudaStream_t stream) {
     static KernelSmemSetup setup;
-    const size_t smem = proj_gemm_smem();
-    cudaError_t e = setup.ensure(proj_gemm_kernel, device, 0, (int)smem);
+    cudaError_t e = setup.ensure(proj_gemm_kernel<BN>, device, 0, (int)GemmGeom<BN>::SMEM);
     if (e != cudaSuccess) return e;
-    dim3 grid((a.N + kGemmBN - 1) / kGemmBN, (a.m + kGemmBM - 1) / kGemmBM);
-    proj_gemm_kernel<<<grid, kGemmThreads, smem, stream>>>(tmA, tmB, a);
-    return cudaGetLastError();
+    int tiles = 0;
+    for (int i = 0; i < a.n_mats; ++i) {
+        a.tile0[i] = tiles;
+        tiles += (a.N[i] + BN - 1) / BN;
+    }
+    return launch_chained(chained, proj_gemm_kernel<BN>, dim3(tiles, (a.m + kGemmBM - 1) / kGemmBM), kGemmThreads,
+                          GemmGeom<BN>::SMEM, stream, tmA, *tmB[0], *tmB[a.n_mats > 1 ? 1 : 0], *tmB[a.n_mats > 2 ? 2 : 0], a);
+}
+
+// Tile width: a 128 x 128 tile takes about 0.6 of the time of a 128 x 256 one (both are fed by the L2: 32 and 48 KB per
+// k-step), so the narrow one pays where it fills SMs that would stay idle and adds no wave.
+inline cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap* const* tmB, const GemmArgs& a, bool chained, int device,
+                               int sm_count, cudaStream_t stream) {
+    const int64_t mt = (a.m + kGemmBM - 1) / kGemmBM;
+    int64_t wide = 0, narrow = 0;
+    for (int i = 0; i < a.n_mats; ++i) {
+        wide += mt * ((a.N[i] + 255) / 256);
+        narrow += mt * ((a.N[i] + 127) / 128);
+    }
+    const int64_t waves_wide = (wide + sm_count - 1) / sm_count, waves_narrow = (narrow + sm_count - 1) / sm_count;
+    return 6 * waves_narrow < 10 * waves_wide ? launch_gemm_inst<128>(tmA, tmB, a, chained, device, stream)
+                                              : launch_gemm_inst<256>(tmA, tmB, a, chained, device, stream);
 }
 
 }  // namespace ggr
