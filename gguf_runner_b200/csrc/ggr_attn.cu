@@ -2282,7 +2282,7 @@ struct ggr_weights {
     __half2* d_dm = nullptr;           // Q4_K: (d, dmin) per super-block [rows][cols / 256]
     float* d_scales_f32 = nullptr;     // Q6_K: d * scale per 16 weights [rows][cols / 16]
     __nv_bfloat16* d_bf16 = nullptr;   // bf16 image for the tensor-core kernel (d_main itself for BF16)
-    CUtensorMap tmB;                   // [rows][cols] bf16, box 64 x 128
+    CUtensorMap tmB;                   // [rows][cols] bf16, box 64 x 64
     bool have_tmap = false;
 };
 

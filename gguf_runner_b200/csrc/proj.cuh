@@ -12,8 +12,8 @@
 //                     d * scale * sum(x q) - dmin * min * sum(x), one FMA per weight) and Q6_K (kept as int8 codes
 //                     q - 32 with one f32 scale per 16 weights, which is one lane's load).
 //   proj_gemm_kernel  prefill chunks: tcgen05 GEMM, bf16 x bf16 -> f32 in TMEM. A = activations [m][K] (bf16), B =
-//                     weights [N][K] (bf16; Q8_0 / F32 weights use a bf16 image made at upload), 128 x 256 or
-//                     128 x 128 output tile per CTA, 64-column k-steps through a four- or six-stage TMA ring, one MMA issuer, four epilogue
+//                     weights [N][K] (bf16; Q8_0 / F32 weights use a bf16 image made at upload), 128 rows x 64
+//                     to 256 columns per CTA, 64-column k-steps through a four- to eight-stage TMA ring, one MMA issuer, four epilogue
 //                     warps reading the accumulator out of TMEM. Every wait is bounded.
 #pragma once
 
@@ -407,12 +407,13 @@ struct GemmArgs {
 };
 
 constexpr int kGemmBM = 128, kGemmBK = 64;
-constexpr int kGemmBoxN = 128;     // weight rows of one TMA box
+constexpr int kGemmBoxN = 64;      // weight rows of one TMA box
 constexpr int kGemmThreads = 192;  // four epilogue warps, a TMA producer, an MMA issuer
 constexpr uint32_t kGemmABytes = kGemmBM * kGemmBK * 2, kGemmBoxBytes = kGemmBoxN * kGemmBK * 2;
 template <int BN>
 struct GemmGeom {
-    static constexpr int STAGES = BN == 256 ? 4 : 6;  // 192 KB either way
+    static constexpr int STAGES = BN == 256 ? 4 : BN == 192 ? 5 : BN == 128 ? 6 : 8;  // 192 to 200 KB
+    static constexpr int TMEM_COLS = BN == 192 ? 256 : BN;  // a power of two
     static constexpr uint32_t BBYTES = BN * kGemmBK * 2;
     static constexpr size_t SMEM = (size_t)STAGES * (kGemmABytes + BBYTES) + 1024;
 };
@@ -447,7 +448,7 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) {
-        tmem_alloc(smem_u32(&s_tmem_base), BN);
+        tmem_alloc(smem_u32(&s_tmem_base), GemmGeom<BN>::TMEM_COLS);
         tmem_relinquish();
     }
     grid_allow_dependents();
@@ -550,11 +551,11 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    if (warp == 5) tmem_dealloc(tmem, BN);
+    if (warp == 5) tmem_dealloc(tmem, GemmGeom<BN>::TMEM_COLS);
     if (tid == 0 && s_abort && a.err) atomicExch(a.err, 1);
 }
 
-// tmA: activations [m][K] with a 64 x 128 box; tmB: weights [N][K] with a 64 x 128 box, one map per matrix
+// tmA: activations [m][K] with a 64 x 128 box; tmB: weights [N][K] with a 64 x 64 box, one map per matrix
 template <int BN>
 inline cudaError_t launch_gemm_inst(const CUtensorMap& tmA, const CUtensorMap* const* tmB, GemmArgs a, bool chained, int device,
                                     cudaStream_t stream) {
@@ -570,19 +571,30 @@ inline cudaError_t launch_gemm_inst(const CUtensorMap& tmA, const CUtensorMap* c
                           GemmGeom<BN>::SMEM, stream, tmA, *tmB[0], *tmB[a.n_mats > 1 ? 1 : 0], *tmB[a.n_mats > 2 ? 2 : 0], a);
 }
 
-// Tile width: a 128 x 128 tile takes about 0.6 of the time of a 128 x 256 one (both are fed by the L2: 32 and 48 KB per
-// k-step), so the narrow one pays where it fills SMs that would stay idle and adds no wave.
+// Tile width: the one with the smallest product of waves and time of a tile. Times relative to 256 columns (K = 4096,
+// measured): 192: 0.85, 128: 0.57; 64: 0.43, from the 48 cycles its MMA takes where the 128-wide one takes 64 (both read A
+// from shared memory).
 inline cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap* const* tmB, const GemmArgs& a, bool chained, int device,
                                int sm_count, cudaStream_t stream) {
+    constexpr int widths[4] = {256, 192, 128, 64}, tile_time[4] = {100, 85, 57, 43};
     const int64_t mt = (a.m + kGemmBM - 1) / kGemmBM;
-    int64_t wide = 0, narrow = 0;
-    for (int i = 0; i < a.n_mats; ++i) {
-        wide += mt * ((a.N[i] + 255) / 256);
-        narrow += mt * ((a.N[i] + 127) / 128);
+    int best = 0;
+    int64_t best_time = -1;
+    for (int w = 0; w < 4; ++w) {
+        int64_t tiles = 0;
+        for (int i = 0; i < a.n_mats; ++i) tiles += mt * ((a.N[i] + widths[w] - 1) / widths[w]);
+        const int64_t t = (tiles + sm_count - 1) / sm_count * tile_time[w];
+        if (best_time < 0 || t < best_time) {
+            best = w;
+            best_time = t;
+        }
     }
-    const int64_t waves_wide = (wide + sm_count - 1) / sm_count, waves_narrow = (narrow + sm_count - 1) / sm_count;
-    return 6 * waves_narrow < 10 * waves_wide ? launch_gemm_inst<128>(tmA, tmB, a, chained, device, stream)
-                                              : launch_gemm_inst<256>(tmA, tmB, a, chained, device, stream);
+    switch (widths[best]) {
+        case 256: return launch_gemm_inst<256>(tmA, tmB, a, chained, device, stream);
+        case 192: return launch_gemm_inst<192>(tmA, tmB, a, chained, device, stream);
+        case 128: return launch_gemm_inst<128>(tmA, tmB, a, chained, device, stream);
+        default: return launch_gemm_inst<64>(tmA, tmB, a, chained, device, stream);
+    }
 }
 
 }  // namespace ggr
