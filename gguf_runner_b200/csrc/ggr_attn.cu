@@ -1105,6 +1105,22 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
                 a.gate_bf16 = in_dtype == GGR_DTYPE_BF16;
                 a.gate_head_stride = gate_head_stride;
             }
+            a.n_split = 1;
+            if (!wide) {
+                int vs, ve, vs1, ve1;
+                visible_host(c, layer, base_pos + i0 + n - 1, &vs, &ve);
+                visible_host(c, layer, std::max(base_pos + i0, base_pos + i0 + n - 2 * kTcBM), &vs1, &ve1);
+                int ns = prefill_tc_splits(n, c->kv.Hq, (std::max(ve, ve1) + kTcBN - 1) / kTcBN - std::min(vs, vs1) / kTcBN, c->sm_count);
+                if (c->cfg.max_splits > 0) ns = std::min(ns, c->cfg.max_splits);
+                if (ns > 1) {
+                    const size_t rows = (size_t)ns * n * c->kv.Hq;
+                    int r = ensure(c, &c->d_part, &c->part_cap, rows * (c->D + 2));
+                    if (r) return r;
+                    a.n_split = ns;
+                    a.part = c->d_part;
+                    a.ml = reinterpret_cast<float2*>(c->d_part + rows * c->D);
+                }
+            }
 #ifdef GGR_TC_TRACE
             a.trace = g_tc_trace;
 #endif

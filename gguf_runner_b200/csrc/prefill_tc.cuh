@@ -31,6 +31,7 @@
 // all roles leave their loops, TMEM is freed and the host sees GGR_ERR_TIMEOUT.
 #pragma once
 
+#include <algorithm>
 #include <string>
 
 #include "common.cuh"
@@ -47,7 +48,13 @@ struct PrefillTcArgs {
     float score_scale;       // (1/sqrt(D) or 1) * log2(e)
     int* err;                // device-visible error word (mapped host memory)
     int* sched;              // [0] work items handed out beyond the first wave, [1] CTAs that have left (persistent kernel)
-    int n_items;             // query-tile pairs x query heads
+    int n_items;             // query-tile pairs x query heads x key splits
+    // Key splits: where the pairs and heads leave half of the SMs idle, an item is one of n_split equal parts of a pair's
+    // key tiles and leaves its un-normalised rows in part [n_split][m][Hq][D] and (maximum, sum) in ml [n_split][m][Hq];
+    // prefill_merge_kernel makes the output.
+    int n_split;
+    float* part;
+    float2* ml;
     // optional output gate (src/engine/runtime/inference.rs:3509-3519), f32 or bf16: head h of row i at
     // gate + (i * Hq + h) * gate_head_stride elements
     const void* gate;
@@ -112,6 +119,7 @@ struct TcItem {
     int h, kvh, q_row0;
     int lo0, hi0, lo1, hi1;  // visible 128-key tiles [lo_t, hi_t) of query tile t (ranges are monotone in the position)
     int lo, hi;              // their union: the key tiles the CTA walks
+    int split;
     __device__ __forceinline__ int lo_of(int t) const { return t ? lo1 : lo0; }
     __device__ __forceinline__ int hi_of(int t) const { return t ? hi1 : hi0; }
     __device__ __forceinline__ bool active(int t, int j) const { return j >= lo_of(t) && j < hi_of(t); }
@@ -122,6 +130,8 @@ __device__ __forceinline__ TcItem tc_item(const PrefillTcArgs& a, int r) {
     TcItem it;
     const int Hq = a.kv.Hq;
     const int n_pairs = (a.m + 2 * kTcBM - 1) / (2 * kTcBM);
+    it.split = r % a.n_split;
+    r /= a.n_split;
     const int pair = n_pairs - 1 - r / Hq;
     it.h = r % Hq;
     it.kvh = it.h / a.kv.G;
@@ -140,6 +150,15 @@ __device__ __forceinline__ TcItem tc_item(const PrefillTcArgs& a, int r) {
         a.vis.range(a.base_pos + r1, vs1, ve1);
         lo_t[t] = min(vs0, vs1) / kTcBN;
         hi_t[t] = (max(ve0, ve1) + kTcBN - 1) / kTcBN;
+    }
+    if (a.n_split > 1) {
+        const int lo = hi_t[1] > lo_t[1] ? min(lo_t[0], lo_t[1]) : lo_t[0], hi = max(hi_t[0], hi_t[1]);
+        const int chunk = (hi - lo + a.n_split - 1) / a.n_split, s_lo = lo + it.split * chunk, s_hi = min(hi, s_lo + chunk);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            lo_t[t] = max(lo_t[t], s_lo);
+            hi_t[t] = max(lo_t[t], min(hi_t[t], s_hi));
+        }
     }
     it.lo0 = lo_t[0], it.hi0 = hi_t[0], it.lo1 = lo_t[1], it.hi1 = hi_t[1];
     const bool act0 = it.hi0 > it.lo0, act1 = it.hi1 > it.lo1;
@@ -220,7 +239,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     volatile int* itemp = s_item;
     const int64_t row_base = a.kv.row(a.seq, a.layer, 0);
     const int Hq = a.kv.Hq;
-    if (a.dependent) asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_allow_dependents();
+    if (a.dependent) grid_wait();
 
     if (warp >= 8) {
       // control warpgroup: gives registers up; warps 10 and 11 have no role
@@ -551,15 +571,20 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             if (!(ok = mbar_wait(o_final(t), it & 1, abortp))) break;
             TRACE_ADD(ts_ofin);
             fence_after_sync();
+            float* orow0 = a.out;
+            if (a.n_split > 1) {
+                orow0 = a.part + (int64_t)w.split * a.m * Hq * D;
+                if (valid) a.ml[((int64_t)w.split * a.m + qi) * Hq + w.h] = make_float2(m_used, l);
+            }
             if (n_t > 0) {
                 // The rows leave through a per-warp staging area: a thread (one query row) lays 32 output columns
                 // down as 128 bytes, 16-byte pieces XOR-swizzled by the row so that the eight rows of a quarter
                 // warp hit different banks; the warp then reads the area back four rows at a time and stores
                 // whole 128-byte lines. One thread per row storing 16-byte pieces 16 KB apart cost a cache-line
                 // wavefront per lane and instruction, 3-4 us per item during which the tile's pipeline stood still.
-                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+                const float inv = a.n_split > 1 ? 1.0f : (l > 0.0f ? 1.0f / l : 0.0f);
                 const void* grow = nullptr;
-                if (a.gate && valid)
+                if (a.gate && valid && a.n_split == 1)
                     grow = static_cast<const unsigned char*>(a.gate) +
                            ((int64_t)qi * Hq + w.h) * a.gate_head_stride * (a.gate_bf16 ? 2 : 4);
                 const uint32_t stage = sOut + (uint32_t)warp * 4096u;
@@ -589,7 +614,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                                      : "=f"(o4.x), "=f"(o4.y), "=f"(o4.z), "=f"(o4.w)
                                      : "r"(stage + rr * 128u + (uint32_t)((piece ^ (rr & 7)) << 4)));
                         if (row_w + rr < a.m)
-                            *reinterpret_cast<float4*>(a.out + ((int64_t)(row_w + rr) * Hq + w.h) * D + cidx * 32 + piece * 4) = o4;
+                            *reinterpret_cast<float4*>(orow0 + ((int64_t)(row_w + rr) * Hq + w.h) * D + cidx * 32 + piece * 4) = o4;
                     }
                     __syncwarp();
                 }
@@ -634,7 +659,48 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
 }
 
+// Merges the key splits of a launch: a thread owns four output elements of one (row, head). Splits without a visible
+// tile left (-infinity, 0) and no rows.
+template <int D>
+__global__ void __launch_bounds__(256) prefill_merge_kernel(PrefillTcArgs a) {
+    grid_allow_dependents();
+    grid_wait();
+    const int64_t rows = (int64_t)a.m * a.kv.Hq, idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t row = idx / (D / 4);
+    const int d = (int)(idx - row * (D / 4)) * 4;
+    if (row >= rows) return;
+    float top = -INFINITY;
+    for (int s = 0; s < a.n_split; ++s) top = fmaxf(top, __ldcg(&a.ml[s * rows + row]).x);
+    float l = 0.0f;
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int s = 0; s < a.n_split; ++s) {
+        const float2 ml = __ldcg(&a.ml[s * rows + row]);
+        if (ml.x == -INFINITY) continue;
+        const float f = exp2f((ml.x - top) * a.score_scale);
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(a.part + (s * rows + row) * D + d));
+        l = fmaf(f, ml.y, l);
+        o.x = fmaf(f, x.x, o.x);
+        o.y = fmaf(f, x.y, o.y);
+        o.z = fmaf(f, x.z, o.z);
+        o.w = fmaf(f, x.w, o.w);
+    }
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    if (a.gate)
+        o = prefill_gate4(o, static_cast<const unsigned char*>(a.gate) + row * a.gate_head_stride * (a.gate_bf16 ? 2 : 4), a.gate_bf16, d);
+    *reinterpret_cast<float4*>(a.out + row * D + d) = o;
+}
+
 // ---- host side ---------------------------------------------------------------------------------
+
+// Key splits of a launch whose longest pair walks `tiles` key tiles: as many as fill the SMs, if they can be filled twice
+// over by splitting, and at least four tiles each (a step over a tile takes about 2 us, the merge 4 to 5).
+// (333 rows behind 1700, 32/8 heads of 128: 64 items of 16 tiles -> 128 of 8, 57 -> 47 us per layer with rope and merge.)
+inline int prefill_tc_splits(int m, int Hq, int tiles, int sm_count) {
+    const int items = (m + 2 * kTcBM - 1) / (2 * kTcBM) * Hq;
+    const int n = std::min(std::min(sm_count / std::max(1, items), tiles / 4), 8);
+    return std::max(1, n);
+}
 
 inline bool prefill_tc_shape_ok(int fmt, int D) { return fmt == KV_BF16 && (D == 64 || D == 128); }
 
@@ -664,7 +730,7 @@ inline int launch_prefill_tc_inst(const CUtensorMap& tq, const CUtensorMap& tk, 
     }
     PrefillTcArgs args = a;
     const int n_pairs = (a.m + 2 * kTcBM - 1) / (2 * kTcBM);
-    args.n_items = n_pairs * a.kv.Hq;
+    args.n_items = n_pairs * a.kv.Hq * a.n_split;
     const int grid = args.n_items < sm_count ? args.n_items : sm_count;  // one persistent CTA per SM
     cudaError_t e;
     if (args.dependent) {
@@ -686,6 +752,14 @@ inline int launch_prefill_tc_inst(const CUtensorMap& tq, const CUtensorMap& tk, 
     if (e != cudaSuccess) {
         *msg = std::string("prefill kernel launch: ") + cudaGetErrorString(e);
         return 2;
+    }
+    if (args.n_split > 1) {
+        const int64_t threads = (int64_t)a.m * a.kv.Hq * (D / 4);
+        e = launch_chained(args.dependent != 0, prefill_merge_kernel<D>, dim3((unsigned)((threads + 255) / 256)), 256, 0, stream, args);
+        if (e != cudaSuccess) {
+            *msg = std::string("prefill merge launch: ") + cudaGetErrorString(e);
+            return 2;
+        }
     }
     return 0;
 }
