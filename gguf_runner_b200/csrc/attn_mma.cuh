@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_mma_decode_kernel(AttnArg
     constexpr int NT = D / 8;    // n-tiles of P.V
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_mma_decode_kernel(AttnArg
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -268,10 +269,11 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_mma_decode_kernel(AttnArg
             wl[warp * 16 + gq + 8] = l1;
         }
         __syncthreads();
-        cta_merge_store(a, wacc, wm, wl, kMmaWarps, 16, g0, min(16, G - g0), item, kvh, split);
+        cta_merge_store(a, wacc, wm, wl, kMmaWarps, 16, g0, min(16, G - g0), sp, kvh);
         __syncthreads();
     }
-    split_merge_store(a, item, kvh, &s_last, reinterpret_cast<float*>(smem));
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem));
 }
 
 template <int D, int NST>
@@ -300,32 +302,35 @@ inline int launch_mma_decode(const AttnArgs& a, dim3 grid, size_t smem, int smem
 // The running output is rescaled only when a row maximum grows by more than 2^8.
 
 constexpr int kTmaTK = 16;
-constexpr int kTmaWarps = 8;
+// Warps per CTA: eight (one CTA per SM: the rings take 196 KB), or four (two CTAs per SM) for ragged batches, where one
+// CTA's prologue and merge then run beside the other's stream (16 sequences of 200 to 6000 keys, 40/8 heads: 40 -> 31 us per layer, prologue of the next
+// layer ahead included).
+constexpr int kTmaWarps = 8, kTmaWarpsRagged = 4;
 constexpr int kTmaNST = 3;
 
 inline bool mma_tma_decode_supported(int D) { return D == 64 || D == 128; }
 
-inline MmaPlan mma_tma_plan(int D, int smem_optin) {
+inline MmaPlan mma_tma_plan(int D, int warps, int smem_optin) {
     MmaPlan p{};
     const int stage = 2 * kTmaTK * D * 2;
     p.nst = kTmaNST;
-    size_t ring = (size_t)kTmaWarps * kTmaNST * stage;
-    size_t merge = (size_t)kTmaWarps * 16 * (D + 8 + 2) * sizeof(float) + 256;
+    size_t ring = (size_t)warps * kTmaNST * stage;
+    size_t merge = (size_t)warps * 16 * (D + 8 + 2) * sizeof(float) + 256;
     p.smem = (ring > merge ? ring : merge) + 1024;  // slack to align the ring to the swizzle atom
     p.ctas_per_sm = (int)((size_t)(smem_optin + 1024) / (p.smem + 4096));
     if (p.ctas_per_sm < 1) p.ctas_per_sm = 1;
     if (p.ctas_per_sm > 4) p.ctas_per_sm = 4;
-    p.min_keys = kTmaWarps * kTmaTK * 2;
+    p.min_keys = warps * kTmaTK * 2;
     return p;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(const __grid_constant__ CUtensorMap tmK,
+template <int D, int W>
+__global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                              const __grid_constant__ CUtensorMap tmV,
                                                                              AttnArgs a) {
     using namespace tc;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(8) uint64_t s_full[kTmaWarps][kTmaNST];
+    __shared__ __align__(8) uint64_t s_full[W][kTmaNST];
     __shared__ int s_last;
     __shared__ int s_abort;
     constexpr int NBLK = D / 64;                   // 64-column (128-byte) blocks of a row
@@ -337,12 +342,13 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
     constexpr int NST = kTmaNST;
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int gq = lane >> 2, tq = lane & 3;
-    peer_allow_dependents(a);
+    if (!a.early) decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -361,7 +367,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
     unsigned char* smem_al = smem + (ring_base - smem_u32(smem));
     const uint32_t ring = ring_base + (uint32_t)warp * NST * STAGE_BYTES;
     const int n_tiles_total = k1 > k0 ? (k1 - k0 + kTmaTK - 1) / kTmaTK : 0;
-    const int my_tiles = n_tiles_total > warp ? (n_tiles_total - warp + kTmaWarps - 1) / kTmaWarps : 0;
+    const int my_tiles = n_tiles_total > warp ? (n_tiles_total - warp + W - 1) / W : 0;
 
     DECODE_STAMP(0);
     if (tid == 0) s_abort = 0;
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
         // one lane: K and V rows [key, key + 16) of this KV head, 64 columns per box
         const uint32_t bar = smem_u32(&s_full[warp][stage]);
         const uint32_t dst = ring + (uint32_t)stage * STAGE_BYTES;
-        const int y = (int)(row0 + k0 + (int64_t)(warp + tile_idx * kTmaWarps) * kTmaTK);
+        const int y = (int)(row0 + k0 + (int64_t)(warp + tile_idx * W) * kTmaTK);
         mbar_expect_tx(bar, STAGE_BYTES);
 #pragma unroll
         for (int b = 0; b < NBLK; ++b) {
@@ -392,11 +398,12 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
     bool prefetched = true;
     if (owner) {
         const int tile_pos = (pos - s0) / kTmaTK;
-        if (tile_pos % kTmaWarps == warp && tile_pos / kTmaWarps < NST - 1) prefetched = false;
+        if (tile_pos % W == warp && tile_pos / W < NST - 1) prefetched = false;
     }
     if (prefetched && lane == 0) {
         for (int s = 0; s < NST - 1 && s < my_tiles; ++s) issue(s, s);
     }
+    if (a.early) decode_begin(a);
     const float* qsrc = a.q + ((int64_t)item * Hq + (int64_t)kvh * G) * D;
     if (a.fused.enabled) qsrc = fused_rope_prologue(a, item, kvh, seq, pos, owner, smem);
     DECODE_STAMP(1);
@@ -439,7 +446,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
             if (!ok) break;
             const uint32_t kt = ring + (uint32_t)stage * STAGE_BYTES;
             const uint32_t vt = kt + MAT_BYTES;
-            const int key0 = k0 + (warp + it * kTmaWarps) * kTmaTK;
+            const int key0 = k0 + (warp + it * W) * kTmaTK;
 
             // S = Q K^T for 16 keys: 2 n-tiles of 8 keys
             float sc[2][4];
@@ -530,8 +537,8 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
         // rows are padded by 8 floats: the eight row groups of a warp then hit different banks
         constexpr int LD = D + 8;
         float* wacc = reinterpret_cast<float*>(smem_al);  // [W][16][LD]
-        float* wm = wacc + kTmaWarps * 16 * LD;
-        float* wl = wm + kTmaWarps * 16;
+        float* wm = wacc + W * 16 * LD;
+        float* wl = wm + W * 16;
         const bool row0_used = g0 + gq < G, row1_used = g0 + gq + 8 < G;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -546,31 +553,33 @@ __global__ void __launch_bounds__(kTmaWarps * 32) attn_mma_tma_decode_kernel(con
             wl[warp * 16 + gq + 8] = l1;
         }
         __syncthreads();
-        cta_merge_store(a, wacc, wm, wl, kTmaWarps, 16, g0, min(16, G - g0), item, kvh, split, LD);
+        cta_merge_store(a, wacc, wm, wl, W, 16, g0, min(16, G - g0), sp, kvh, LD);
         __syncthreads();
     }
     if (tid == 0 && s_abort && a.err) atomicExch(a.err, 1);
     DECODE_STAMP(3);
-    split_merge_store(a, item, kvh, &s_last, reinterpret_cast<float*>(smem_al));
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem_al));
     DECODE_STAMP(4);
 }
 
-template <int D>
+template <int D, int W>
 inline int launch_mma_tma_inst(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid, size_t smem,
                                int smem_optin, int device, cudaStream_t stream) {
     static KernelSmemSetup setup;
-    const cudaError_t se = setup.ensure(attn_mma_tma_decode_kernel<D>, device, smem_optin);
+    const cudaError_t se = setup.ensure(attn_mma_tma_decode_kernel<D, W>, device, smem_optin);
     if (se != cudaSuccess) return (int)se;
-    attn_mma_tma_decode_kernel<D><<<grid, kTmaWarps * 32, smem, stream>>>(tk, tv, a);
-    return (int)cudaGetLastError();
+    return (int)launch_chained(a.chained, attn_mma_tma_decode_kernel<D, W>, grid, W * 32, smem, stream, tk, tv, a);
 }
 
 // tk / tv: tensor maps over the whole K and V arrays with a box of 64 columns x 16 rows
-inline int launch_mma_tma_decode(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid, size_t smem,
-                                 int smem_optin, int device, cudaStream_t stream) {
+inline int launch_mma_tma_decode(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, int warps, dim3 grid,
+                                 size_t smem, int smem_optin, int device, cudaStream_t stream) {
     switch (a.kv.D) {
-        case 64: return launch_mma_tma_inst<64>(tk, tv, a, grid, smem, smem_optin, device, stream);
-        case 128: return launch_mma_tma_inst<128>(tk, tv, a, grid, smem, smem_optin, device, stream);
+        case 64: return warps == kTmaWarps ? launch_mma_tma_inst<64, kTmaWarps>(tk, tv, a, grid, smem, smem_optin, device, stream)
+                                           : launch_mma_tma_inst<64, kTmaWarpsRagged>(tk, tv, a, grid, smem, smem_optin, device, stream);
+        case 128: return warps == kTmaWarps ? launch_mma_tma_inst<128, kTmaWarps>(tk, tv, a, grid, smem, smem_optin, device, stream)
+                                            : launch_mma_tma_inst<128, kTmaWarpsRagged>(tk, tv, a, grid, smem, smem_optin, device, stream);
         default: return (int)cudaErrorNotSupported;
     }
 }

@@ -62,6 +62,8 @@ struct AttnArgs {
     float* partial_out;   // [items][Hq][D + 2] (o / l, m, l) for cross-rank merging, or null
     int shard_count;      // positions held locally
     int stage_bytes;      // bytes of one ring stage of one warp
+    int chained;          // launched programmatically behind the kernel in front (launch_chained)
+    int early;            // the kernel in front writes no cache row of this layer: the first tiles may be requested at once
     int tile_stages;      // ring stages of the CTA-tile kernel (1 or 2)
     int* err;             // raised when a bounded wait runs out (kernels that wait on mbarriers)
     FusedRope fused;
@@ -74,6 +76,31 @@ struct AttnArgs {
     long long* trace;     // per-CTA phase time stamps (diagnostic builds only)
 #endif
 };
+
+// Which item and which of its n splits a CTA works on; state of (head h, split s): row first + h * n + s of a.part.
+struct SplitPos {
+    int item, split, n;
+    int64_t first;
+};
+__device__ __forceinline__ SplitPos split_pos(const AttnArgs& a) {
+    SplitPos sp;
+    if (a.items.ragged) {
+        int lo = 0, hi = a.items.n - 1;  // the last item that starts at or before this split
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.items.split0[mid] <= blockIdx.x)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        lo = __shfl_sync(0xffffffffu, lo, 0);  // (tells the compiler that the result is warp-uniform)
+        const int s0 = a.items.split0[lo];
+        sp = SplitPos{lo, (int)blockIdx.x - s0, a.items.split0[lo + 1] - s0, (int64_t)s0 * a.kv.Hq};
+    } else {
+        sp = SplitPos{(int)blockIdx.z, (int)blockIdx.x, a.n_split, (int64_t)blockIdx.z * a.kv.Hq * a.n_split};
+    }
+    return sp;
+}
 
 // phase time stamps of diagnostic builds: slot k of this CTA's row in a.trace
 #ifdef GGR_TC_TRACE
@@ -285,9 +312,9 @@ __device__ __forceinline__ void store_final(const AttnArgs& a, int item, int h, 
 // wm / wl [nw][RS]) for heads g0 .. g0+gn-1 of this KV head and stores them: final
 // when the launch has one split, else into the split scratch.
 __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* wacc, float* wm, float* wl, int nw,
-                                                int RS, int g0, int gn, int item, int kvh, int split, int ld = 0) {
+                                                int RS, int g0, int gn, const SplitPos& sp, int kvh, int ld = 0) {
     if (ld == 0) ld = a.kv.D;  // row stride of wacc (the tensor-core kernels pad it against bank conflicts)
-    const int D = a.kv.D, G = a.kv.G, Hq = a.kv.Hq;
+    const int D = a.kv.D, G = a.kv.G;
     // one thread per head turns the warps' maxima into weights once (wm <- 2^(m_w - max), wl[g] <- merged l,
     // wx[g] <- max), so the per-element loop below is a plain weighted sum
     float* wx = wl + nw * RS;
@@ -311,10 +338,10 @@ __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* 
         for (int w = 0; w < nw; ++w) o = fmaf(wm[w * RS + g], wacc[(w * RS + g) * ld + d], o);
         const float ms = wx[g], ls = wl[g];
         const int h = kvh * G + g0 + g;
-        if (a.n_split == 1) {
-            store_final(a, item, h, d, o, ms, ls);
+        if (sp.n == 1) {
+            store_final(a, sp.item, h, d, o, ms, ls);
         } else {
-            float* pp = a.part + (((int64_t)item * Hq + h) * a.n_split + split) * (D + 2);
+            float* pp = a.part + (sp.first + (int64_t)h * sp.n + sp.split) * (D + 2);
             pp[d] = o;
             if (d == 0) {
                 pp[D] = ms;
@@ -324,11 +351,16 @@ __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* 
     }
 }
 
-// Start of a kernel that feeds the fused shard exchange: lets the merge kernel enqueued behind it (launched with
-// programmatic stream serialisation) become resident once every CTA of this grid has started, so that its launch
-// and its wait for the peers' flags overlap this grid's work. A no-op for every other launch.
-__device__ __forceinline__ void peer_allow_dependents(const AttnArgs& a) {
-    if (a.px.enabled) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// Decode kernels are launched behind each other (launch_chained): decode_begin waits for the kernel in front. The next
+// one is let in by decode_tail, when every CTA of this grid has reached its merge; its first tiles (AttnArgs::early) then
+// travel while the last CTAs merge. The merge kernel of the fused shard exchange is small and is let in at once: its
+// launch and its wait for the peers' flags overlap this grid's work.
+__device__ __forceinline__ void decode_begin(const AttnArgs& a) {
+    if (a.px.enabled) grid_allow_dependents();
+    grid_wait();
+}
+__device__ __forceinline__ void decode_tail(const AttnArgs& a) {
+    if (!a.px.enabled) grid_allow_dependents();
 }
 
 // Called by the CTA that stored the final states of a (token, kv head) group. When every group of the
@@ -360,12 +392,13 @@ inline size_t split_merge_sub_floats(int G, int D) { return G <= 4 ? (size_t)G *
 // The last CTA of a (token, kv head) to arrive (atomic ticket) merges the
 // per-split states from the scratch buffer and resets the ticket. `wsm` is
 // shared memory for G * n_split weights (the drained ring is reused).
-__device__ __forceinline__ void split_merge_store(const AttnArgs& a, int item, int kvh, int* s_last, float* wsm) {
-    if (a.n_split == 1) {
+__device__ __forceinline__ void split_merge_store(const AttnArgs& a, const SplitPos& sp, int kvh, int* s_last, float* wsm) {
+    const int item = sp.item;
+    if (sp.n == 1) {
         peer_group_done(a);
         return;
     }
-    const int D = a.kv.D, G = a.kv.G, Hq = a.kv.Hq, NS = a.n_split;
+    const int D = a.kv.D, G = a.kv.G, NS = sp.n;
     // one fence on each side of the ticket, issued by the thread that takes it: the CTA barrier before it orders
     // every thread's stores of this CTA's state ahead of the fence, the barrier after it orders every thread's
     // loads of the other CTAs' states behind it (fences are cumulative)
@@ -379,7 +412,7 @@ __device__ __forceinline__ void split_merge_store(const AttnArgs& a, int item, i
     __syncthreads();
     if (!*s_last) return;
     DECODE_STAMP(5);
-    const float* base = a.part + ((int64_t)item * Hq + (int64_t)kvh * G) * NS * (D + 2);
+    const float* base = a.part + (sp.first + (int64_t)kvh * G * NS) * (D + 2);
     // One warp per head; this CTA runs alone at the end of the launch and a round trip to the states that other
     // SMs just wrote costs about 1.4 us, so everything is arranged for few dependent round trips: (m, l) of all
     // splits in one lane-strided batch of 8-byte loads, the split outputs in batches of 16 or 32 independent
@@ -617,14 +650,15 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_simt_kernel(AttnArgs a) 
     __shared__ int s_last;
 
     const int D = a.kv.D, G = a.kv.G, Hq = a.kv.Hq;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nw = blockDim.x >> 5;  // 1, 2 or 4 warps, each with its own ring
     const int rowbytes = D * a.kv.elem_bytes;
     DECODE_STAMP(0);
-    peer_allow_dependents(a);
+    decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -634,7 +668,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_simt_kernel(AttnArgs a) 
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);  // cache row of local position 0
@@ -805,12 +839,13 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_simt_kernel(AttnArgs a) 
             }
         }
         __syncthreads();
-        cta_merge_store(a, wacc, wm, wl, nw, GH, g0, min(GH, G - g0), item, kvh, split);
+        cta_merge_store(a, wacc, wm, wl, nw, GH, g0, min(GH, G - g0), sp, kvh);
         __syncthreads();  // merge area is free again before the next head group refills the ring
     }
 
     DECODE_STAMP(3);
-    split_merge_store(a, item, kvh, &s_last, reinterpret_cast<float*>(smem));
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem));
     DECODE_STAMP(4);
 }
 
@@ -924,6 +959,7 @@ __global__ void combine_exchange_kernel(const float* parts, const int* flags, in
             *reinterpret_cast<float2*>(out + ((int64_t)item * Hq + h) * D + 2 * db) = make_float2(rx, ry);
         }
     }
+    grid_wait();  // this grid is done only when the send kernel in front is: what follows waits for this grid alone
 }
 
 }  // namespace ggr

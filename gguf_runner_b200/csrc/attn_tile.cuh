@@ -66,11 +66,12 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
     __shared__ int s_last;
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nst = a.tile_stages;
     DECODE_STAMP(0);
-    peer_allow_dependents(a);
+    if (!a.early) decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
             cp_async_commit();
         }
     }
+    if (a.early) decode_begin(a);
     const float* qsrc = a.q + ((int64_t)item * Hq + (int64_t)kvh * G) * D;
     if (a.fused.enabled) qsrc = fused_rope_prologue(a, item, kvh, seq, pos, owner, smem);
     DECODE_STAMP(1);
@@ -318,10 +320,10 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
 #pragma unroll
                 for (int q = 0; q < KG; ++q) o += red[((size_t)q * gh + g) * D + d];
                 const int h = kvh * G + g0 + g;
-                if (a.n_split == 1) {
+                if (sp.n == 1) {
                     store_final(a, item, h, d, o, m_s[g], l_s[g]);
                 } else {
-                    float* pp = a.part + (((int64_t)item * Hq + h) * a.n_split + split) * (D + 2);
+                    float* pp = a.part + (sp.first + (int64_t)h * sp.n + split) * (D + 2);
                     pp[d] = o;
                     if (d == 0) {
                         pp[D] = m_s[g];
@@ -337,10 +339,10 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
 #pragma unroll
                     for (int e = 0; e < EPT; ++e) {
                         const int d = dt * EPT + e;
-                        if (a.n_split == 1) {
+                        if (sp.n == 1) {
                             store_final(a, item, h, d, acc[g][e], m_s[g], l_s[g]);
                         } else {
-                            float* pp = a.part + (((int64_t)item * Hq + h) * a.n_split + split) * (D + 2);
+                            float* pp = a.part + (sp.first + (int64_t)h * sp.n + split) * (D + 2);
                             pp[d] = acc[g][e];
                             if (d == 0) {
                                 pp[D] = m_s[g];
@@ -353,7 +355,8 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
         __syncthreads();  // the ring is free again before the next head group refills it
     }
     DECODE_STAMP(3);
-    split_merge_store(a, item, kvh, &s_last, reinterpret_cast<float*>(smem));
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem));
     DECODE_STAMP(4);
 }
 
@@ -403,8 +406,7 @@ inline int launch_tile_inst(const AttnArgs& a, dim3 grid, size_t smem, int smem_
     static KernelSmemSetup setup;
     const cudaError_t se = setup.ensure(attn_tile_kernel<FMT, D>, device, smem_optin);
     if (se != cudaSuccess) return (int)se;
-    attn_tile_kernel<FMT, D><<<grid, kTileThreads, smem, stream>>>(a);
-    return (int)cudaGetLastError();
+    return (int)launch_chained(a.chained, attn_tile_kernel<FMT, D>, grid, kTileThreads, smem, stream, a);
 }
 
 template <int FMT>

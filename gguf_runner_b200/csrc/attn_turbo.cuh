@@ -78,6 +78,8 @@ struct TurboAppendArgs {
 // grid (items, Hkv), 64 threads: warp 0 quantises the K head, warp 1 the V head (:885-952)
 __global__ void __launch_bounds__(64) turbo_append_kernel(TurboAppendArgs a) {
     extern __shared__ float tsm[];
+    grid_wait();
+    grid_allow_dependents();
     const int D = a.kv.D, kv_dim = a.kv.kv_dim;
     const int item = blockIdx.x, kvh = blockIdx.y, lane = threadIdx.x & 31, which = threadIdx.x >> 5;
     int seq, pos;
@@ -158,7 +160,8 @@ __global__ void __launch_bounds__(kTurboWarps * 32) attn_turbo_kernel(AttnArgs a
     constexpr int CB = EPL / 4;    // code bytes per lane
     constexpr int SB = EPL / 8;    // sign bytes per lane
     const int G = a.kv.G, Hkv = a.kv.Hkv, kv_dim = a.kv.kv_dim;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int grp = warp * 4 + (lane >> 3), sl = lane & 7;
     const unsigned gmask = 0xffu << (lane & 24);
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kTurboWarps * 32) attn_turbo_kernel(AttnArgs a
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk, s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
     const int k0 = s0 - a.kv.pos_begin, k1 = s1 - a.kv.pos_begin;
@@ -326,10 +329,11 @@ __global__ void __launch_bounds__(kTurboWarps * 32) attn_turbo_kernel(AttnArgs a
         }
         __syncthreads();
         // one un-normalised state per head goes to the output, the cross-rank partial or the split scratch
-        cta_merge_store(a, fin, wm, wl, 1, GH, g0, min(GH, G - g0), item, kvh, split, 2 * D);
+        cta_merge_store(a, fin, wm, wl, 1, GH, g0, min(GH, G - g0), sp, kvh, 2 * D);
         __syncthreads();
     }
-    split_merge_store(a, item, kvh, &s_last, work);
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, work);
 }
 
 template <int D, int GH>

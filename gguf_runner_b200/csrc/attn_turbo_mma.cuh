@@ -134,9 +134,11 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     __shared__ int s_last;
     constexpr int D = kTmD, KS = D / 16, NT = D / 8, rowbytes = D * 2;
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const int split = blockIdx.x, kvh = blockIdx.y, item = blockIdx.z;
+    const SplitPos sp = split_pos(a);
+    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int gq = lane >> 2, tq = lane & 3;
+    decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -145,7 +147,7 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + a.n_split - 1) / a.n_split;
+    const int chunk = (T + sp.n - 1) / sp.n;
     const int s0 = vs + split * chunk, s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
     const int k0 = s0 - a.kv.pos_begin, k1 = s1 - a.kv.pos_begin;
@@ -378,17 +380,17 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
         sm_[16 + tid] = tid < G ? hm[16 + tid] : 0.0f;
     }
     __syncthreads();
-    cta_merge_store(a, fin, sm_, sm_ + 16, 1, 16, 0, G, item, kvh, split, 2 * D);
+    cta_merge_store(a, fin, sm_, sm_ + 16, 1, 16, 0, G, sp, kvh, 2 * D);
     __syncthreads();
-    split_merge_store(a, item, kvh, &s_last, reinterpret_cast<float*>(tsm8));
+    decode_tail(a);
+    split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(tsm8));
 }
 
 inline int launch_turbo_mma(const AttnArgs& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
     static KernelSmemSetup setup;
     const cudaError_t se = setup.ensure(attn_turbo_mma_kernel, device, smem_optin);
     if (se != cudaSuccess) return (int)se;
-    attn_turbo_mma_kernel<<<grid, kTmWarps * 32, smem, stream>>>(a);
-    return (int)cudaGetLastError();
+    return (int)launch_chained(a.chained, attn_turbo_mma_kernel, grid, kTmWarps * 32, smem, stream, a);
 }
 
 }  // namespace ggr

@@ -82,6 +82,10 @@ struct Items {
     int mode;  // 0: decode, item b -> (seq b, pos[b]); 1: prefill, item i -> (seq0, base_pos + i)
     int seq0, base_pos, n;
     int pos[kMaxArgItems];
+    // Sequences of different lengths (decode only): item i is split split0[i + 1] - split0[i] ways, and the splits of
+    // all items are numbered one after the other in blockIdx.x. Otherwise every item is split the same way.
+    int ragged;
+    unsigned short split0[kMaxArgItems + 1];
 
     __device__ __forceinline__ void get(int item, int& seq, int& p) const {
         if (mode == 0) {
@@ -176,6 +180,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // the launch, the CTA start-up and what does not depend on the predecessor (barriers, tensor memory, weights) cost no
 // time of their own. Every kernel launched that way calls grid_wait() before it touches memory that any earlier work
 // in the stream may write or read; that covers work of other origin too, since the predecessor has waited likewise.
+// grid_allow_dependents() comes after grid_wait(): whatever runs ahead of its own grid_wait() can then only meet the one
+// kernel in front of it (the merge kernel of the shard exchange apart, which reads nothing but what flags guard).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -89,6 +89,7 @@ struct ggr_attn_ctx {
     // error word the kernels raise when a bounded wait runs out (mapped pinned host memory)
     int* h_err = nullptr;
     int* d_err = nullptr;
+    int tail_layer = -1;     // layer whose cache rows the last appending launch wrote; -1: unknown
     int* d_sched = nullptr;  // work counters of the persistent prefill kernel (rewound by the kernel itself)
     // per-layer pre-attention fixups (device arrays, null = absent) and their f32 scratch rows
     struct LayerFixups {
@@ -283,7 +284,7 @@ int ensure_copy_streams(ggr_attn_ctx* c, int n_pieces) {
 
 // Applies the layer's bias / QK-norm fixups to n rows of q/k/v (device memory, element type es bytes)
 // and redirects the pointers to the f32 scratch rows. No-op for layers without fixups.
-int apply_fixups(ggr_attn_ctx* c, int layer, int n, const void** q, const void** k, const void** v, int* in_bf16) {
+int apply_fixups(ggr_attn_ctx* c, int layer, int n, const void** q, const void** k, const void** v, int* in_bf16, bool chain) {
     if ((size_t)layer >= c->fixups.size() || !c->fixups[layer].any()) return GGR_OK;
     const auto& f = c->fixups[layer];
     int rc;
@@ -319,9 +320,8 @@ int apply_fixups(ggr_attn_ctx* c, int layer, int n, const void** q, const void**
         b.v_out = a.v_out + (size_t)i0 * c->kv_dim;
         {
             LaunchTimer t(c, 1);
-            qkv_fixup_kernel<<<cnt, 256, 0, c->stream>>>(b);
+            CUDA_TRY(c, launch_chained(chain && chain_launches(c), qkv_fixup_kernel, dim3(cnt), 256, 0, c->stream, b));
         }
-        CUDA_TRY(c, cudaGetLastError());
         c->launches++;
     }
     *q = c->d_fix[0];
@@ -340,6 +340,7 @@ int check_layer(ggr_attn_ctx* c, int layer) {
 
 int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags, int in_bf16, const void* q,
                        const void* k, const void* v, float* q_out, __nv_bfloat16* q_out_h, float* k_out) {
+    if (flags & RF_APPEND) c->tail_layer = layer;
     RopeAppendArgs a{};
     a.rope = rope_params(c, layer);
     a.kv = c->kv;
@@ -356,7 +357,7 @@ int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags
     a.shard_count = c->shard_count;
     // TurboQuant: the rope kernel leaves the rotated keys in a scratch buffer and a second kernel quantises
     // them and the values head by head
-    const bool turbo = c->kv.fmt == KV_TURBO;
+    const bool turbo = c->kv.fmt == KV_TURBO, chained = chain_launches(c);
     const bool turbo_append = turbo && (flags & RF_APPEND);
     const float* turbo_k = nullptr;
     bool skip_rope = false;
@@ -378,18 +379,16 @@ int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags
     }
     if (!skip_rope) {
         LaunchTimer t(c, 1);
-        if (turbo)
-            rope_append_kernel<<<items.n, 256, smem, c->stream>>>(a);
-        else if (rope_append_fast_ok(a))
-            rope_append_bf16_kernel<<<items.n, 256, 0, c->stream>>>(a);
-        else if (rope_append_vec_ok(a) && smem + 16 <= 48 * 1024 && in_bf16)
-            rope_append_vec_kernel<__nv_bfloat16><<<items.n, 256, smem + 16, c->stream>>>(a);
-        else if (rope_append_vec_ok(a) && smem + 16 <= 48 * 1024)
-            rope_append_vec_kernel<float><<<items.n, 256, smem + 16, c->stream>>>(a);
-        else
-            rope_append_kernel<<<items.n, 256, smem, c->stream>>>(a);
+        auto kernel = rope_append_kernel;
+        if (!turbo && rope_append_fast_ok(a)) {
+            kernel = rope_append_bf16_kernel;
+            smem = 0;
+        } else if (!turbo && rope_append_vec_ok(a) && smem + 16 <= 48 * 1024) {
+            kernel = in_bf16 ? rope_append_vec_kernel<__nv_bfloat16> : rope_append_vec_kernel<float>;
+            smem += 16;
+        }
+        CUDA_TRY(c, launch_chained(chained && items.mode == 0, kernel, dim3(items.n), 256, smem, c->stream, a));
     }
-    CUDA_TRY(c, cudaGetLastError());
     if (!skip_rope) c->launches++;
     if (turbo_append) {
         TurboAppendArgs t{};
@@ -402,9 +401,9 @@ int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags
         t.shard_count = c->shard_count;
         {
             LaunchTimer lt(c, 1);
-            turbo_append_kernel<<<dim3(items.n, c->kv.Hkv), 64, (size_t)4 * c->D * sizeof(float), c->stream>>>(t);
+            CUDA_TRY(c, launch_chained(chained, turbo_append_kernel, dim3(items.n, c->kv.Hkv), 64, (size_t)4 * c->D * sizeof(float),
+                                       c->stream, t));
         }
-        CUDA_TRY(c, cudaGetLastError());
         c->launches++;
     }
     return GGR_OK;
@@ -487,21 +486,44 @@ int launch_simt(ggr_attn_ctx* c, const AttnArgs& a, dim3 grid, const SimtPlan& p
     }
 }
 
+// Visible lengths of the sequences of a decode call.
+struct Lengths {
+    int n = 0, len[kMaxArgItems];
+    bool ragged() const { return n > 1 && *std::min_element(len, len + n) != *std::max_element(len, len + n); }
+    // splits of all items when the longest (t_max keys) is split `splits` ways and the others into pieces of that size
+    int total(int t_max, int splits) const {
+        const int chunk = (t_max + splits - 1) / splits;
+        int sum = 0;
+        for (int i = 0; i < n; ++i) sum += std::max(1, (len[i] + chunk - 1) / chunk);
+        return sum;
+    }
+    // numbers the splits in `items`
+    void number(int t_max, int splits, Items* items) const {
+        const int chunk = (t_max + splits - 1) / splits;
+        items->ragged = 1;
+        items->split0[0] = 0;
+        for (int i = 0; i < n; ++i)
+            items->split0[i + 1] = (unsigned short)(items->split0[i] + std::max(1, (len[i] + chunk - 1) / chunk));
+    }
+};
+
 // Split-KV factor. The grid is base_ctas * n CTAs running `slots` at a time, each CTA streaming
 // ceil(T / n) keys of `bytes_per_key` bytes. A wave of c concurrent CTAs moves data at
 // min(per-CTA rate, HBM rate / c) per CTA and costs a fixed start/finish time; merging n splits
 // costs a little per split. The constants are measured on B200 (TMA-fed decode kernel: ~65 GB/s per
-// CTA alone, ~6.6 TB/s for the whole GPU, ~8 us per wave). Picks the n with the smallest modelled time.
+// CTA alone, ~6.6 TB/s for the whole GPU, ~8 us per wave). Picks the n with the smallest modelled time. For a ragged
+// batch n is the split count of the longest sequence, and base_ctas counts the CTAs of one split of one sequence.
 int choose_splits(int64_t base_ctas, int64_t slots, int t_max, int min_keys, int max_splits, double bytes_per_key,
-                  double cta_rate, double t_wave = 8e-6) {
+                  double cta_rate, double t_wave = 8e-6, const Lengths* ragged = nullptr) {
     int limit = std::max(1, t_max / std::max(1, min_keys));
-    limit = std::min(limit, 512);
+    limit = std::min(limit, ragged ? 511 : 512);  // (511 * kMaxArgItems splits still fit Items::split0)
     if (max_splits > 0) limit = std::min(limit, max_splits);
     const double hbm_rate = 6.6e12;
     int best = 1;
     double best_cost = -1.0;
-    for (int n = 1; n <= limit; ++n) {
-        const int64_t ctas = base_ctas * n;
+    const int step = ragged ? std::max(1, limit * ragged->n / 4096) : 1;  // (bounds the host time of a call)
+    for (int n = 1; n <= limit; n += step) {
+        const int64_t ctas = base_ctas * (ragged ? ragged->total(t_max, n) : n);
         const int64_t full = ctas / slots, rem = ctas % slots;
         const double bytes = (double)((t_max + n - 1) / n) * bytes_per_key;
         double cost = 0.0;
@@ -539,7 +561,17 @@ struct DecodePlan {
     size_t smem;
     int ctas_per_sm, min_keys;
     double cta_rate;
+    int warps;  // of the TMA-fed tensor-core kernel
 };
+
+void use_tma_plan(const ggr_attn_ctx* c, DecodePlan& d, int warps) {
+    const MmaPlan mp = mma_tma_plan(c->D, warps, c->smem_optin);
+    d.warps = warps;
+    d.smem = mp.smem;
+    d.ctas_per_sm = mp.ctas_per_sm;
+    d.min_keys = mp.min_keys;
+    d.cta_rate = warps == kTmaWarps ? 65e9 : 35e9;
+}
 
 void use_tile_plan(const ggr_attn_ctx* c, DecodePlan& d, int nst) {
     d.tp = tile_plan(c->kv.fmt, c->D, nst, c->smem_optin);
@@ -557,9 +589,11 @@ DecodePlan decode_plan(const ggr_attn_ctx* c, bool allow_mma) {
     d.smem = d.p.smem;
     d.ctas_per_sm = d.p.ctas_per_sm;
     d.min_keys = d.p.nw * kSimtTK * 2;
-    d.cta_rate = d.tma ? 65e9 : 40e9;
-    if (d.mma) {
-        MmaPlan mp = d.tma ? mma_tma_plan(c->D, c->smem_optin) : mma_plan(c->D, c->smem_optin);
+    d.cta_rate = 40e9;
+    if (d.tma) {
+        use_tma_plan(c, d, kTmaWarps);
+    } else if (d.mma) {
+        const MmaPlan mp = mma_plan(c->D, c->smem_optin);
         d.smem = mp.smem;
         d.ctas_per_sm = mp.ctas_per_sm;
         d.min_keys = mp.min_keys;
@@ -573,10 +607,10 @@ DecodePlan decode_plan(const ggr_attn_ctx* c, bool allow_mma) {
 
 // Split-KV factor of a launch. The CTA-tile kernel streams with one ring stage when every CTA gets a single tile
 // and with two otherwise, which changes its occupancy and so the split count: settle both here.
-int plan_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits) {
+int plan_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits, const Lengths* ragged = nullptr) {
     auto pick = [&]() {
-        return choose_splits((int64_t)c->kv.Hkv * n_items, (int64_t)c->sm_count * d.ctas_per_sm, t_max, d.min_keys,
-                             max_splits, 2.0 * c->D * c->kv.elem_bytes, d.cta_rate, d.tile ? 3e-6 : 8e-6);
+        return choose_splits((int64_t)c->kv.Hkv * (ragged ? 1 : n_items), (int64_t)c->sm_count * d.ctas_per_sm, t_max, d.min_keys,
+                             max_splits, 2.0 * c->D * c->kv.elem_bytes, d.cta_rate, d.tile ? 3e-6 : 8e-6, ragged);
     };
     int n = pick();
     if (d.tile && ((t_max + n - 1) / n + d.tp.tk - 1) / d.tp.tk > 1) {
@@ -616,12 +650,26 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     a.out = out_dev;
     a.partial_out = partial_dev;
     a.shard_count = c->shard_count;
+    a.chained = chain_launches(c);
     if (px) a.px = *px;
     a.err = c->d_err;
     if (gate && gate->p) {
         a.gate = static_cast<const float*>(gate->p);  // callers hand f32 gates to this path
         a.gate_head_stride = gate->head_stride;
     }
+
+    // Decode of sequences of different lengths: pieces of one size instead of one number of pieces, so that no CTA has
+    // more to do than another. (16 sequences of 200 to 6000 keys, 40/8 heads of 128, bf16: 45 -> 31 us per layer.)
+    Lengths lengths;
+    if (items.mode == 0 && items.n > 1) {
+        for (int i = 0; i < items.n; ++i) {
+            int vs, ve;
+            visible_host(c, layer, items.pos[i], &vs, &ve);
+            lengths.len[i] = std::max(0, std::min(ve, c->shard_begin + c->shard_count) - std::max(vs, c->shard_begin));
+        }
+        lengths.n = items.n;
+    }
+    bool ragged = lengths.ragged();
 
     if (c->kv.fmt == KV_TURBO) {
         // TurboQuant cache: rope + quantising append as separate launches, then the CUDA-core attention kernel.
@@ -648,7 +696,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             double best_eff = -1.0;
             n_split = 1;
             for (int n = 1; n <= limit; ++n) {
-                const int64_t ctas = base_ctas * n, waves = (ctas + c->sm_count - 1) / c->sm_count;
+                const int64_t ctas = ragged ? (int64_t)c->kv.Hkv * lengths.total(t_max, n) : base_ctas * n, waves = (ctas + c->sm_count - 1) / c->sm_count;
                 const double eff = (double)ctas / (double)(waves * c->sm_count);
                 if (eff > best_eff + 1e-9) {
                     best_eff = eff;
@@ -658,10 +706,14 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             }
         }
         n_split = std::min(n_split, limit);
+        ragged = ragged && tc && n_split > 1;
+        if (ragged) lengths.number(t_max, n_split, &a.items);
+        const int total = ragged ? a.items.split0[items.n] : items.n * n_split;
+        const dim3 grid = ragged ? dim3(total, c->kv.Hkv, 1) : dim3(n_split, c->kv.Hkv, items.n);
         a.n_split = n_split;
         c->last_splits = n_split;
         if (n_split > 1) {
-            int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)items.n * c->kv.Hq * n_split * (c->D + 2));
+            int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)total * c->kv.Hq * (c->D + 2));
             if (rc) return rc;
             const size_t before = c->counters_cap;
             rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)items.n * c->kv.Hkv);
@@ -676,13 +728,13 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             const size_t smem = turbo_mma_smem_bytes(c->G, n_split);
             a.stage_bytes = (int)turbo_mma_prep_offset(c->G, n_split);
             LaunchTimer t(c, 0);
-            e = launch_turbo_mma(a, dim3(n_split, c->kv.Hkv, items.n), smem, c->smem_optin, c->cfg.device, c->stream);
+            e = launch_turbo_mma(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         } else {
             const size_t smem = turbo_attn_smem_floats(c->D, c->G, turbo_heads_per_pass(c->G, c->D), n_split) * sizeof(float);
             if (smem + 1024 > (size_t)c->smem_optin)
                 return fail(c, GGR_ERR_UNSUPPORTED, "TurboQuant attention: too many query heads per KV head for shared memory");
             LaunchTimer t(c, 0);
-            e = launch_turbo_attention(a, dim3(n_split, c->kv.Hkv, items.n), smem, c->smem_optin, c->cfg.device, c->stream);
+            e = launch_turbo_attention(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (e != 0) return fail(c, GGR_ERR_CUDA, std::string("TurboQuant attention launch: ") + cudaGetErrorString((cudaError_t)e));
         c->launches++;
@@ -690,8 +742,14 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     }
 
     DecodePlan dp = decode_plan(c, allow_mma);
-    int n_split = plan_splits(c, dp, items.n, t_max, c->cfg.max_splits);
-    {
+    ragged = ragged && (dp.tma || dp.tile);
+    if (ragged && dp.tma) use_tma_plan(c, dp, kTmaWarpsRagged);
+    int n_split = plan_splits(c, dp, items.n, t_max, c->cfg.max_splits, ragged ? &lengths : nullptr);
+    if (ragged) {
+        const size_t fit = c->part_cap / ((size_t)c->kv.Hq * (c->D + 2));  // splits of all items the reservation holds
+        while (c->reserved_batch > 0 && n_split > 1 && (size_t)lengths.total(t_max, n_split) > fit) --n_split;
+        ragged = n_split > 1;
+    } else {
         // with a reservation in place the split count never outgrows the reserved scratch (as long as that
         // holds two splits): the decode loop then neither allocates nor synchronises for memory
         const size_t per_split = (size_t)items.n * c->kv.Hq * (c->D + 2);
@@ -729,8 +787,14 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         }
     }
 
+    // The rows of other layers were complete before the kernel in front began, so the loads of the first tiles overlap
+    // its tail (its split merge, mostly).
+    a.early = a.chained && a.fused.enabled && !px && c->tail_layer >= 0 && c->tail_layer != layer;
+    if (raw) c->tail_layer = px ? -1 : layer;  // (the send kernel of the exchange lets the next one in before it waits itself)
     a.n_split = n_split;
     c->last_splits = n_split;
+    if (ragged) lengths.number(t_max, n_split, &a.items);
+    const int total_splits = ragged ? a.items.split0[items.n] : items.n * n_split;
     // the split merge stages one weight per (head, split) in shared memory
     const size_t merge_smem = split_merge_smem_bytes(c, n_split);
     smem = std::max(smem, merge_smem);
@@ -742,7 +806,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         smem = p.smem = (size_t)a.fused.smem_off + fb;
     }
     if (n_split > 1) {
-        int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)items.n * c->kv.Hq * n_split * (c->D + 2));
+        int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)total_splits * c->kv.Hq * (c->D + 2));
         if (rc) return rc;
         const size_t before = c->counters_cap;
         rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)items.n * c->kv.Hkv);
@@ -752,7 +816,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         a.part = c->d_part;
         a.counters = c->d_counters;
     }
-    dim3 grid(n_split, c->kv.Hkv, items.n);
+    const dim3 grid = ragged ? dim3(total_splits, c->kv.Hkv, 1) : dim3(n_split, c->kv.Hkv, items.n);
 #ifdef GGR_TC_TRACE
     a.trace = g_tc_trace;
 #endif
@@ -760,7 +824,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         int rc;
         {
             LaunchTimer t(c, 0);
-            rc = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, grid, smem, c->smem_optin, c->cfg.device, c->stream)
+            rc = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, dp.warps, grid, smem, c->smem_optin, c->cfg.device, c->stream)
                      : launch_mma_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (rc != 0) return fail(c, GGR_ERR_CUDA, std::string("mma decode launch: ") + cudaGetErrorString((cudaError_t)rc));
@@ -793,6 +857,7 @@ int launch_split_prefill(ggr_attn_ctx* c, int layer, const Items& items, int t_m
     a.score_scale = (c->cfg.scale_mode == GGR_SCALE_SCORE ? c->attn_scale : 1.0f) * kLog2e;
     a.out = out_dev;
     a.shard_count = c->shard_count;
+    a.chained = chain_launches(c);
     if (gate.p) {
         a.gate = static_cast<const float*>(gate.p);
         a.gate_head_stride = gate.head_stride;
@@ -882,7 +947,7 @@ constexpr size_t kZeroCopyOutBytes = 64 * 1024;
 int reserve_decode(ggr_attn_ctx* c, int B) {
     int rc;
     if ((rc = ensure(c, &c->d_qrot, &c->qrot_cap, (size_t)B * c->q_dim))) return rc;
-    int splits = 1;
+    int splits = 1, ragged_rows = 0;
     if (c->kv.fmt == KV_TURBO) {
         splits = c->cfg.max_splits > 0 ? std::min(64, c->cfg.max_splits) : 64;
         if ((rc = ensure(c, &c->d_krot, &c->krot_cap, (size_t)B * c->kv_dim))) return rc;
@@ -894,10 +959,15 @@ int reserve_decode(ggr_attn_ctx* c, int B) {
             splits = std::max(splits, plan_splits(c, dp, chunk, t, c->cfg.max_splits));
             if (t == 1) break;
         }
+        // a ragged batch in up to two waves of CTAs
+        DecodePlan dp = decode_plan(c, true);
+        if (dp.tma) use_tma_plan(c, dp, kTmaWarpsRagged);
+        if (chunk > 1) ragged_rows = 2 * c->sm_count * dp.ctas_per_sm / c->kv.Hkv + chunk;
     }
     const int chunk = std::min(B, kMaxArgItems);
-    if (splits > 1) {
-        if ((rc = ensure(c, &c->d_part, &c->part_cap, (size_t)chunk * c->kv.Hq * splits * (c->D + 2)))) return rc;
+    if (splits > 1 || ragged_rows > 0) {
+        const size_t rows = std::max(chunk * splits, ragged_rows);
+        if ((rc = ensure(c, &c->d_part, &c->part_cap, rows * c->kv.Hq * (c->D + 2)))) return rc;
         const size_t before = c->counters_cap;
         if ((rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)chunk * c->kv.Hkv))) return rc;
         if (c->counters_cap != before)
@@ -961,7 +1031,7 @@ int decode_common(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const f
     }
     if ((rc = ensure(c, &c->d_qrot, &c->qrot_cap, (size_t)B * c->q_dim))) return rc;
     int in_bf16 = 0;
-    if ((rc = apply_fixups(c, layer, B, &dq, &dk, &dv, &in_bf16))) return rc;
+    if ((rc = apply_fixups(c, layer, B, &dq, &dk, &dv, &in_bf16, true))) return rc;
 
     for (int b0 = 0; b0 < B; b0 += kMaxArgItems) {
         const int n = std::min(kMaxArgItems, B - b0);
@@ -1073,7 +1143,7 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
             const void* fk = dk + (size_t)j0 * c->kv_dim * es;
             const void* fv = dv + (size_t)j0 * c->kv_dim * es;
             int in_bf16 = in_dtype == GGR_DTYPE_BF16;
-            int r = apply_fixups(c, layer, cnt, &fq, &fk, &fv, &in_bf16);
+            int r = apply_fixups(c, layer, cnt, &fq, &fk, &fv, &in_bf16, false);
             if (r) return r;
             r = launch_rope_append(c, layer, it, RF_ROTATE | RF_WRITE_Q | RF_APPEND, in_bf16, fq, fk, fv,
                                    tc ? nullptr : c->d_qrot + (size_t)j0 * c->q_dim,
@@ -2030,7 +2100,7 @@ extern "C" int ggr_attn_attention_tokens_static(ggr_attn_ctx* c, int32_t layer, 
         int e;
         {
             LaunchTimer t(c, 0);
-            e = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, grid, smem, c->smem_optin, c->cfg.device, c->stream)
+            e = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, dp.warps, grid, smem, c->smem_optin, c->cfg.device, c->stream)
                     : launch_mma_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (e != 0) return fail(c, GGR_ERR_CUDA, std::string("mma decode launch: ") + cudaGetErrorString((cudaError_t)e));
@@ -2135,7 +2205,7 @@ int exchange_send(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const f
     if ((rc = stage_in(c, 2, v, kb, ptr_kind, &dv))) return rc;
     if ((rc = ensure(c, &c->d_qrot, &c->qrot_cap, (size_t)B * c->q_dim))) return rc;
     int in_bf16 = 0;
-    if ((rc = apply_fixups(c, layer, B, &dq, &dk, &dv, &in_bf16))) return rc;
+    if ((rc = apply_fixups(c, layer, B, &dq, &dk, &dv, &in_bf16, true))) return rc;
     const int n = c->cfg.n_ranks, me = c->cfg.rank;
     // the step counter moves only once the kernel is in the stream: a send that fails on the host leaves the
     // ranks' counters in agreement
@@ -2407,7 +2477,7 @@ int matmul_device(ggr_attn_ctx* c, const ggr_weights* w, const float* x, int n, 
         fill_gemv(a, w, x, n, out, ld_out, sanitize);
         {
             LaunchTimer t(c, 3);
-            CUDA_TRY(c, launch_gemv(w->wtype, a, c->cfg.device, c->sm_count, c->stream));
+            CUDA_TRY(c, launch_gemv(w->wtype, a, chain_launches(c), c->cfg.device, c->sm_count, c->stream));
         }
         c->launches++;
         return GGR_OK;
@@ -2670,7 +2740,7 @@ extern "C" int ggr_attn_layer_decode(ggr_attn_ctx* c, int32_t layer, const int32
         }
         {
             LaunchTimer t(c, 3);
-            CUDA_TRY(c, launch_gemv(wq->wtype, a, c->cfg.device, c->sm_count, c->stream));
+            CUDA_TRY(c, launch_gemv(wq->wtype, a, chain_launches(c), c->cfg.device, c->sm_count, c->stream));
         }
         c->launches++;
     } else {

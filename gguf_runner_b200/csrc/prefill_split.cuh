@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(PsLayout<FMT, D>::threads, PsLayout<FMT, D>::c
     const int n_rows = a.items.n * G, r_first = row_tile * kPsRows;
     const int seq = a.items.seq0;
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
+    grid_wait();
+    grid_allow_dependents();
 
     if (tid == 0) {
         s_lo = INT_MAX;
@@ -566,8 +568,7 @@ inline cudaError_t launch_prefill_split_inst(const AttnArgs& a, dim3 grid, int s
     static KernelSmemSetup setup;
     const cudaError_t e = setup.ensure(prefill_split_kernel<FMT, D>, device, smem_optin, PsLayout<FMT, D>::bytes);
     if (e != cudaSuccess) return e;
-    prefill_split_kernel<FMT, D><<<grid, PsLayout<FMT, D>::threads, PsLayout<FMT, D>::bytes, stream>>>(a);
-    return cudaGetLastError();
+    return launch_chained(a.chained, prefill_split_kernel<FMT, D>, grid, PsLayout<FMT, D>::threads, PsLayout<FMT, D>::bytes, stream, a);
 }
 
 inline cudaError_t launch_prefill_split(const AttnArgs& a, dim3 grid, int smem_optin, int device, cudaStream_t stream) {

@@ -239,8 +239,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     volatile int* itemp = s_item;
     const int64_t row_base = a.kv.row(a.seq, a.layer, 0);
     const int Hq = a.kv.Hq;
-    grid_allow_dependents();
     if (a.dependent) grid_wait();
+    grid_allow_dependents();
 
     if (warp >= 8) {
       // control warpgroup: gives registers up; warps 10 and 11 have no role
@@ -663,8 +663,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // tile left (-infinity, 0) and no rows.
 template <int D>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(PrefillTcArgs a) {
-    grid_allow_dependents();
     grid_wait();
+    grid_allow_dependents();
     const int64_t rows = (int64_t)a.m * a.kv.Hq, idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int64_t row = idx / (D / 4);
     const int d = (int)(idx - row * (D / 4)) * 4;

@@ -194,8 +194,13 @@ __global__ void __launch_bounds__(kGemvWarps * 32, (TT == 1 || WT == PW_F32 || W
     };
 
     for (int t0 = 0; t0 < a.n; t0 += TT) {
-        // the first unit's weights are requested before the activation rows are staged: both latencies overlap
+        // the first unit's weights are requested before the activation rows are staged, and on the first pass before the
+        // kernel that makes these rows has finished: the latencies overlap
         if (n_units > 0) load_unit(0, ba);
+        if (t0 == 0) {
+            grid_wait();
+            grid_allow_dependents();
+        }
         __syncthreads();  // every warp is done with the rows of the previous pass
         // A lane multiplies CPL consecutive columns per step, i.e. CPL / 4 float4 pieces that lie 4 * CPL bytes apart
         // from its neighbour's: read straight, that is a 4-way (Q8_0) or 2-way bank conflict on every load. The rows
@@ -204,7 +209,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, (TT == 1 || WT == PW_F32 || W
         for (int i4 = threadIdx.x; i4 < TT * c4n; i4 += kGemvWarps * 32) {
             const int t = i4 / c4n, col4 = i4 - t * c4n;
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (t0 + t < a.n) v = __ldg(reinterpret_cast<const float4*>(a.x + (size_t)(t0 + t) * cols) + col4);
+            if (t0 + t < a.n) v = *(reinterpret_cast<const float4*>(a.x + (size_t)(t0 + t) * cols) + col4);
             const int step = col4 / (32 * Q), ln = (col4 % (32 * Q)) / Q, q = col4 % Q;
             reinterpret_cast<float4*>(xs)[(size_t)t * row4 + (step * Q + q) * 32 + ln] = v;
         }
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, (TT == 1 || WT == PW_F32 || W
 constexpr int kGemvMaxCols = 12288;  // activation rows are staged in shared memory: up to 48 KB per row
 
 template <int WT, int TT>
-inline cudaError_t launch_gemv_inst(const GemvArgs& a, int device, int sm_count, cudaStream_t stream) {
+inline cudaError_t launch_gemv_inst(const GemvArgs& a, bool chained, int device, int sm_count, cudaStream_t stream) {
     static KernelSmemSetup setup;
     const size_t smem = (size_t)TT * gemv_row_floats<WT>(a.cols) * sizeof(float);
     cudaError_t e = setup.ensure(proj_gemv_kernel<WT, TT>, device, 0, (int)((size_t)TT * gemv_row_floats<WT>(kGemvMaxCols) * sizeof(float)));
@@ -351,31 +356,30 @@ inline cudaError_t launch_gemv_inst(const GemvArgs& a, int device, int sm_count,
     const int groups = ((a.n_extra > 0 ? a.rows_all : a.rows) + kGemvWarps * kGemvRPW - 1) / (kGemvWarps * kGemvRPW);
     // row groups are dealt round robin to a grid that fills the SMs about twice (the staged rows are loaded once per CTA)
     const int grid = groups < 2 * sm_count ? groups : 2 * sm_count;
-    proj_gemv_kernel<WT, TT><<<grid, kGemvWarps * 32, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_chained(chained, proj_gemv_kernel<WT, TT>, dim3(grid), kGemvWarps * 32, smem, stream, a);
 }
 
 template <int WT>
-inline cudaError_t launch_gemv_wt(const GemvArgs& a, int device, int sm_count, cudaStream_t stream) {
-    if (a.n == 1) return launch_gemv_inst<WT, 1>(a, device, sm_count, stream);
-    if (a.n == 2) return launch_gemv_inst<WT, 2>(a, device, sm_count, stream);
-    return launch_gemv_inst<WT, 4>(a, device, sm_count, stream);
+inline cudaError_t launch_gemv_wt(const GemvArgs& a, bool chained, int device, int sm_count, cudaStream_t stream) {
+    if (a.n == 1) return launch_gemv_inst<WT, 1>(a, chained, device, sm_count, stream);
+    if (a.n == 2) return launch_gemv_inst<WT, 2>(a, chained, device, sm_count, stream);
+    return launch_gemv_inst<WT, 4>(a, chained, device, sm_count, stream);
 }
 
-inline cudaError_t launch_gemv(int wtype, const GemvArgs& a, int device, int sm_count, cudaStream_t stream) {
+inline cudaError_t launch_gemv(int wtype, const GemvArgs& a, bool chained, int device, int sm_count, cudaStream_t stream) {
     switch (wtype) {
-        case PW_F32: return launch_gemv_wt<PW_F32>(a, device, sm_count, stream);
-        case PW_BF16: return launch_gemv_wt<PW_BF16>(a, device, sm_count, stream);
-        case PW_Q4_K: return launch_gemv_wt<PW_Q4_K>(a, device, sm_count, stream);
-        case PW_Q6_K: return launch_gemv_wt<PW_Q6_K>(a, device, sm_count, stream);
-        default: return launch_gemv_wt<PW_Q8_0>(a, device, sm_count, stream);
+        case PW_F32: return launch_gemv_wt<PW_F32>(a, chained, device, sm_count, stream);
+        case PW_BF16: return launch_gemv_wt<PW_BF16>(a, chained, device, sm_count, stream);
+        case PW_Q4_K: return launch_gemv_wt<PW_Q4_K>(a, chained, device, sm_count, stream);
+        case PW_Q6_K: return launch_gemv_wt<PW_Q6_K>(a, chained, device, sm_count, stream);
+        default: return launch_gemv_wt<PW_Q8_0>(a, chained, device, sm_count, stream);
     }
 }
 
 // f32 rows -> bf16 rows (activations on their way into the tensor-core GEMM)
 __global__ void proj_to_bf16_kernel(const float* src, __nv_bfloat16* dst, size_t n) {
-    grid_allow_dependents();
     grid_wait();
+    grid_allow_dependents();
     for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (size_t)gridDim.x * blockDim.x * 4) {
         if (i + 4 <= n) {
             const float4 v = *reinterpret_cast<const float4*>(src + i);
@@ -451,7 +455,6 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_alloc(smem_u32(&s_tmem_base), GemmGeom<BN>::TMEM_COLS);
         tmem_relinquish();
     }
-    grid_allow_dependents();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -478,7 +481,8 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // the weights of the first stages do not depend on the kernel in front, which makes the activations
             const int ahead = min(nk, STAGES);
             for (int k = 0; k < ahead; ++k) load_b(k);
-            grid_wait();
+            grid_wait();  // (here and below: the bounded waits on the barriers start when the kernel in front is done)
+            grid_allow_dependents();
             for (int k = 0; k < nk; ++k) {
                 const int s = k % STAGES;
                 if (k >= ahead) {
@@ -493,6 +497,8 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint64_t dA = smem_desc(sA, 16, 1024), dB = smem_desc(sB, 16, 1024);
         const uint32_t tm = __shfl_sync(0xffffffffu, s_tmem_base, 0);
         bool ok = true;
+        grid_wait();
+        grid_allow_dependents();
         for (int k = 0; k < nk && ok; ++k) {
             const int s = k % STAGES;
             if (!(ok = mbar_wait_warp(full(s), (k / STAGES) & 1, abortp))) break;
@@ -509,6 +515,8 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __nv_bfloat16* const out_h = mat == 2 ? a.out_h[2] : mat == 1 ? a.out_h[1] : a.out_h[0];
         // epilogue: thread = output row of the tile (TMEM lane), 32 columns per tcgen05.ld
         const int row = m0 + warp * 32 + lane;
+        grid_wait();
+        grid_allow_dependents();
         if (mbar_wait(acc_full, 0, abortp)) {
             fence_after_sync();
             const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16);
