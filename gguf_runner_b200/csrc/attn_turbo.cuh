@@ -54,6 +54,36 @@ __device__ __forceinline__ void turbo_transform_warp(float* x, int n, const unsi
     __syncwarp();
 }
 
+// sign_b . FWHT(sign_a . x) of 128 floats, lane i of the warp holding elements 4 i .. 4 i + 3: the additions of
+// turbo_transform_warp in the same order
+__device__ __forceinline__ void turbo_transform_regs(float (&x)[4], const unsigned char* first, const unsigned char* second,
+                                                     int lane) {
+    const int sh = (lane & 1) * 4;
+    const unsigned fa = first[lane >> 1] >> sh, fb = second[lane >> 1] >> sh;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = (fa >> k) & 1 ? -x[k] : x[k];
+    float a = __fadd_rn(x[0], x[1]), b = __fsub_rn(x[0], x[1]), c = __fadd_rn(x[2], x[3]), d = __fsub_rn(x[2], x[3]);
+    x[0] = __fadd_rn(a, c);
+    x[1] = __fadd_rn(b, d);
+    x[2] = __fsub_rn(a, c);
+    x[3] = __fsub_rn(b, d);
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+        const bool upper = lane & w;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float o = __shfl_xor_sync(0xffffffffu, x[k], w);
+            x[k] = upper ? __fsub_rn(o, x[k]) : __fadd_rn(x[k], o);
+        }
+    }
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(128.0f));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x[k] = __fmul_rn(x[k], scale);
+        x[k] = (fb >> k) & 1 ? -x[k] : x[k];
+    }
+}
+
 // sqrt(sum x^2), summed in index order by lane 0 (src/engine/kernels/math.rs:467-473) and broadcast
 __device__ __forceinline__ float turbo_l2_norm_warp(const float* x, int n, int lane) {
     float r = 0.0f;
@@ -63,6 +93,20 @@ __device__ __forceinline__ float turbo_l2_norm_warp(const float* x, int n, int l
         r = __fsqrt_rn(ss);
     }
     return __shfl_sync(0xffffffffu, r, 0);
+}
+
+// the same of 128 floats by all lanes: four of them per (broadcast) load, so that only the additions wait for each other
+__device__ __forceinline__ float turbo_l2_norm_128(const float* x) {
+    float ss = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < 128; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(x + i);
+        ss = __fadd_rn(ss, __fmul_rn(v.x, v.x));
+        ss = __fadd_rn(ss, __fmul_rn(v.y, v.y));
+        ss = __fadd_rn(ss, __fmul_rn(v.z, v.z));
+        ss = __fadd_rn(ss, __fmul_rn(v.w, v.w));
+    }
+    return __fsqrt_rn(ss);
 }
 
 struct TurboAppendArgs {
@@ -75,9 +119,52 @@ struct TurboAppendArgs {
     int shard_count;
 };
 
+// One head of 128 by one warp, four elements per lane: both transforms in registers, the same rounded operations in the
+// same order as turbo_append_kernel's. Bound by the two sums over 128 elements, whose order the format fixes.
+__device__ __forceinline__ void turbo_append_128(const KvView& kv, int layer, int which, int kvh, int lane, int64_t row, float (&x)[4],
+                                                 float* buf) {
+    float r[4];
+    turbo_transform_regs(x, turbo_sign_slot(kv, 0, layer, kvh), turbo_sign_slot(kv, 1, layer, kvh), lane);
+    *reinterpret_cast<float4*>(buf + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+    __syncwarp();
+    const float sigma = __fdiv_rn(turbo_l2_norm_128(buf), __fsqrt_rn(128.0f));
+    const int64_t eo = row * kv.kv_dim + (int64_t)kvh * 128, aux = row * kv.Hkv + kvh;
+    unsigned char* base = reinterpret_cast<unsigned char*>(which == 0 ? kv.k : kv.v) + eo / 4;
+    unsigned char* sign = (which == 0 ? kv.k_sign : kv.v_sign) + eo / 8;
+    if (lane == 0) (which == 0 ? kv.ks : kv.vs)[aux] = sigma;
+    unsigned packed = 0, bits = 0xf;
+    float gamma = 0.0f;
+    if (sigma != 0.0f) {
+        const float inv_sigma = __fdiv_rn(1.0f, sigma);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float t = __fmul_rn(x[k], inv_sigma);
+            const int code = t < -kTurboThreshold ? 0 : (t < 0.0f ? 1 : (t < kTurboThreshold ? 2 : 3));
+            r[k] = __fsub_rn(x[k], __fmul_rn(kTurboCentroid[code], sigma));
+            packed |= (unsigned)code << (2 * k);
+        }
+        __syncwarp();
+        *reinterpret_cast<float4*>(buf + 4 * lane) = make_float4(r[0], r[1], r[2], r[3]);
+        __syncwarp();
+        gamma = turbo_l2_norm_128(buf);
+        if (gamma != 0.0f) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] = __fdiv_rn(r[k], gamma);
+            turbo_transform_regs(r, turbo_sign_slot(kv, 2, layer, kvh), turbo_sign_slot(kv, 3, layer, kvh), lane);
+            bits = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bits |= (r[k] >= 0.0f ? 1u : 0u) << k;
+        }
+    }
+    base[lane] = (unsigned char)packed;
+    const unsigned next = __shfl_down_sync(0xffffffffu, bits, 1);
+    if ((lane & 1) == 0) sign[lane >> 1] = (unsigned char)(bits | next << 4);
+    if (lane == 0) (which == 0 ? kv.k_rn : kv.v_rn)[aux] = gamma;
+}
+
 // grid (items, Hkv), 64 threads: warp 0 quantises the K head, warp 1 the V head (:885-952)
 __global__ void __launch_bounds__(64) turbo_append_kernel(TurboAppendArgs a) {
-    extern __shared__ float tsm[];
+    extern __shared__ __align__(16) float tsm[];
     grid_wait();
     grid_allow_dependents();
     const int D = a.kv.D, kv_dim = a.kv.kv_dim;
@@ -88,6 +175,13 @@ __global__ void __launch_bounds__(64) turbo_append_kernel(TurboAppendArgs a) {
     float* rot = tsm + which * 2 * D;
     float* res = rot + D;
     const int64_t in_off = (int64_t)item * kv_dim + (int64_t)kvh * D;
+    if (D == 128) {
+        float x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = which == 0 ? a.k_rot[in_off + 4 * lane + k] : load_in(a.v, in_off + 4 * lane + k, a.v_bf16);
+        turbo_append_128(a.kv, a.layer, which, kvh, lane, a.kv.row(seq, a.layer, pos), x, rot);
+        return;
+    }
     for (int i = lane; i < D; i += 32) rot[i] = which == 0 ? a.k_rot[in_off + i] : load_in(a.v, in_off + i, a.v_bf16);
     __syncwarp();
     turbo_transform_warp(rot, D, turbo_sign_slot(a.kv, 0, a.layer, kvh), turbo_sign_slot(a.kv, 1, a.layer, kvh), lane);
@@ -135,6 +229,96 @@ __global__ void __launch_bounds__(64) turbo_append_kernel(TurboAppendArgs a) {
         for (int k = 0; k < 8; ++k) bits |= (res[8 * b + k] >= 0.0f ? 1u : 0u) << k;
         sign[b] = (unsigned char)bits;
     }
+}
+
+// Everything between the projections and the attention of a TurboQuant cache with heads of 128, all rotated: biases and
+// QK-norm (qkv_fixup_kernel), RoPE and pre-scale (rope_append_kernel), quantising append (turbo_append_kernel) with the
+// operations of those kernels in their order, so that the cache rows and the rotated queries keep their bits. One warp
+// per head of q, k or v, its four elements per lane in registers throughout: one launch of many small CTAs where a
+// token took three launches, two of them of a single CTA (32/4 heads, QK-norm, one token: 18 + 14 + 12 -> 7 us in ncu).
+struct TurboPrepArgs {
+    RopeParams rope;
+    KvView kv;
+    Items items;
+    int layer, shard_count, in_bf16;
+    const void* q;  // [items][q_dim], f32 or bf16
+    const void* k;  // [items][kv_dim]
+    const void* v;
+    float* q_out;   // [items][q_dim] rotated queries
+    const float *q_bias, *k_bias, *v_bias, *q_norm, *k_norm;  // null: none
+    float eps;
+};
+constexpr int kTurboPrepWarps = 4;
+
+__global__ void __launch_bounds__(kTurboPrepWarps * 32) turbo_prep_kernel(TurboPrepArgs a) {
+    __shared__ __align__(16) float buf[kTurboPrepWarps][128];
+    grid_wait();
+    grid_allow_dependents();
+    constexpr int D = 128;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, item = blockIdx.y;
+    const int hh = blockIdx.x * kTurboPrepWarps + warp, Hq = a.kv.Hq, Hkv = a.kv.Hkv;
+    if (hh >= Hq + 2 * Hkv) return;
+    const int kind = hh < Hq ? 0 : (hh < Hq + Hkv ? 1 : 2);  // q, k, v
+    const int h = kind == 0 ? hh : (kind == 1 ? hh - Hq : hh - Hq - Hkv);
+    int seq, pos;
+    a.items.get(item, seq, pos);
+    const void* src = kind == 0 ? a.q : (kind == 1 ? a.k : a.v);
+    const float* bias = kind == 0 ? a.q_bias : (kind == 1 ? a.k_bias : a.v_bias);
+    const float* norm = kind == 0 ? a.q_norm : (kind == 1 ? a.k_norm : nullptr);
+    const int64_t base = ((int64_t)item * (kind == 0 ? Hq : Hkv) + h) * D;
+    float x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x[k] = load_in(src, base + 4 * lane + k, a.in_bf16);
+        if (bias) x[k] = __fadd_rn(x[k], bias[h * D + 4 * lane + k]);
+    }
+    if (norm) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = lane + 32 * k;  // the summation order of qkv_fixup_kernel
+            float y = load_in(src, base + j, a.in_bf16);
+            if (bias) y = __fadd_rn(y, bias[h * D + j]);
+            ss = fmaf(y, y, ss);
+        }
+        ss = warp_sum(ss);
+        const float inv = 1.0f / sqrtf(ss / (float)D + a.eps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = __fmul_rn(norm[4 * lane + k], __fmul_rn(inv, x[k]));
+    }
+    if (kind < 2) {
+        const bool neox = a.rope.style == 0;
+        float cs[4], sn[4], r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!neox && (k & 1)) {  // adjacent elements share their angle
+                cs[k] = cs[k - 1];
+                sn[k] = sn[k - 1];
+                continue;
+            }
+            const int i = neox ? (4 * lane + k) & 63 : 2 * lane + (k >> 1);
+            const int axis = rope_axis(a.rope.layout, i, a.rope.sections);
+            int coord = pos;
+            if (a.rope.has_plan) coord = pos < a.rope.plan_len ? a.rope.plan[pos * 3 + axis] : a.rope.next_text + (pos - a.rope.plan_len);
+            const float val = __fmul_rn(__fmul_rn((float)coord, a.rope.freqs[i]), a.rope.fscale);
+            sincosf(val, &sn[k], &cs[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float o = neox ? __shfl_xor_sync(0xffffffffu, x[k], 16) : x[k ^ 1];
+            const bool upper = neox ? lane >= 16 : (k & 1);
+            const float v0 = upper ? o : x[k], v1 = upper ? x[k] : o;
+            r[k] = upper ? __fadd_rn(__fmul_rn(v0, sn[k]), __fmul_rn(v1, cs[k])) : __fsub_rn(__fmul_rn(v0, cs[k]), __fmul_rn(v1, sn[k]));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = kind == 0 && a.rope.do_prescale ? __fmul_rn(r[k], a.rope.q_prescale) : r[k];
+    }
+    if (kind == 0) {
+        *reinterpret_cast<float4*>(a.q_out + base + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+        return;
+    }
+    if (pos < a.kv.pos_begin || pos >= a.kv.pos_begin + a.shard_count) return;  // another rank owns this row
+    turbo_append_128(a.kv, a.layer, kind - 1, h, lane, a.kv.row(seq, a.layer, pos), x, buf[warp]);
 }
 
 constexpr int kTurboWarps = 4;

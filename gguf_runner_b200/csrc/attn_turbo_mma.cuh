@@ -176,12 +176,15 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     const unsigned char* res_post = turbo_sign_slot(a.kv, 3, a.layer, kvh);
     const float* qsrc = a.q + ((int64_t)item * Hq + (int64_t)kvh * G) * D;
     for (int g = warp; g < 16; g += kTmWarps) {
-        for (int i = lane; i < D; i += 32) qr[g * D + i] = g < G ? qsrc[(int64_t)g * D + i] : 0.0f;
-        __syncwarp();
-        if (g < G) turbo_transform_warp(qr + g * D, D, rot_pre, rot_post, lane);
-        for (int i = lane; i < D; i += 32) qp[g * D + i] = qr[g * D + i];
-        __syncwarp();
-        if (g < G) turbo_transform_warp(qp + g * D, D, res_pre, res_post, lane);
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        if (g < G) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] = qsrc[(int64_t)g * D + 4 * lane + k];
+            turbo_transform_regs(x, rot_pre, rot_post, lane);
+        }
+        *reinterpret_cast<float4*>(qr + g * D + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+        if (g < G) turbo_transform_regs(x, res_pre, res_post, lane);
+        *reinterpret_cast<float4*>(qp + g * D + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
     }
     __syncthreads();
 
@@ -366,10 +369,18 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     // final transforms (:1323-1334): res <- T(res; res_post, res_pre); base += res; out = T(base; rot_post, rot_pre)
     for (int g = warp; g < G; g += kTmWarps) {
         float* fb = fin + g * 2 * D;
-        turbo_transform_warp(fb + D, D, res_post, res_pre, lane);
-        for (int i = lane; i < D; i += 32) fb[i] = fb[i] + fb[D + i];
-        __syncwarp();
-        turbo_transform_warp(fb, D, rot_post, rot_pre, lane);
+        float x[4], y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            x[k] = fb[4 * lane + k];
+            y[k] = fb[D + 4 * lane + k];
+        }
+        turbo_transform_regs(y, res_post, res_pre, lane);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] += y[k];
+        turbo_transform_regs(x, rot_post, rot_pre, lane);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) fb[4 * lane + k] = x[k];
     }
     __syncthreads();
     // one un-normalised state per head goes to the output, the cross-rank partial or the split scratch; the

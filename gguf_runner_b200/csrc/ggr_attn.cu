@@ -89,6 +89,7 @@ struct ggr_attn_ctx {
     // error word the kernels raise when a bounded wait runs out (mapped pinned host memory)
     int* h_err = nullptr;
     int* d_err = nullptr;
+    bool host_call = false;  // the decode call in progress has host pointers: copies stand between its kernels
     int tail_layer = -1;     // layer whose cache rows the last appending launch wrote; -1: unknown
     int* d_sched = nullptr;  // work counters of the persistent prefill kernel (rewound by the kernel itself)
     // per-layer pre-attention fixups (device arrays, null = absent) and their f32 scratch rows
@@ -236,10 +237,10 @@ void visible_host(const ggr_attn_ctx* c, int layer, int pos, int* vs, int* ve) {
     *ve = e;
 }
 
-// Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, and not
-// into a stream capture, where the node in front may be a copy or an event of the caller's.
+// Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, not
+// where copies stand between them (the attribute then only costs host time), and not into a stream capture, where the node in front may be a copy or an event of the caller's.
 bool chain_launches(const ggr_attn_ctx* c) {
-    if (c->timing) return false;
+    if (c->timing || c->host_call) return false;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
         cudaGetLastError();
@@ -282,10 +283,14 @@ int ensure_copy_streams(ggr_attn_ctx* c, int n_pieces) {
     return GGR_OK;
 }
 
+// TurboQuant caches whose heads are 128 wide and rotated as a whole: one kernel does fixups, RoPE and append
+bool use_turbo_prep(const ggr_attn_ctx* c) { return c->kv.fmt == KV_TURBO && c->D == 128 && c->rope_dim == 128; }
+
 // Applies the layer's bias / QK-norm fixups to n rows of q/k/v (device memory, element type es bytes)
 // and redirects the pointers to the f32 scratch rows. No-op for layers without fixups.
 int apply_fixups(ggr_attn_ctx* c, int layer, int n, const void** q, const void** k, const void** v, int* in_bf16, bool chain) {
     if ((size_t)layer >= c->fixups.size() || !c->fixups[layer].any()) return GGR_OK;
+    if (use_turbo_prep(c)) return GGR_OK;  // done by launch_rope_append
     const auto& f = c->fixups[layer];
     int rc;
     if ((rc = ensure(c, &c->d_fix[0], &c->fix_cap[0], (size_t)n * c->q_dim))) return rc;
@@ -341,6 +346,37 @@ int check_layer(ggr_attn_ctx* c, int layer) {
 int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags, int in_bf16, const void* q,
                        const void* k, const void* v, float* q_out, __nv_bfloat16* q_out_h, float* k_out) {
     if (flags & RF_APPEND) c->tail_layer = layer;
+    if (use_turbo_prep(c) && flags == (RF_ROTATE | RF_WRITE_Q | RF_APPEND)) {
+        TurboPrepArgs p{};
+        p.rope = rope_params(c, layer);
+        p.kv = c->kv;
+        p.items = items;
+        p.layer = layer;
+        p.shard_count = c->shard_count;
+        p.in_bf16 = in_bf16;
+        p.q = q;
+        p.k = k;
+        p.v = v;
+        p.q_out = q_out;
+        if ((size_t)layer < c->fixups.size() && c->fixups[layer].any()) {
+            const auto& f = c->fixups[layer];
+            p.q_bias = f.q_bias;
+            p.k_bias = f.k_bias;
+            p.v_bias = f.v_bias;
+            p.q_norm = f.q_norm;
+            p.k_norm = f.k_norm;
+            p.eps = f.eps > 0.0f ? f.eps : 1e-5f;  // src/engine/runtime/inference.rs:2539-2543
+        }
+        const int heads = c->kv.Hq + 2 * c->kv.Hkv;
+        {
+            LaunchTimer t(c, 1);
+            CUDA_TRY(c, launch_chained(chain_launches(c) && items.mode == 0, turbo_prep_kernel,
+                                       dim3((heads + kTurboPrepWarps - 1) / kTurboPrepWarps, items.n), kTurboPrepWarps * 32, 0,
+                                       c->stream, p));
+        }
+        c->launches++;
+        return GGR_OK;
+    }
     RopeAppendArgs a{};
     a.rope = rope_params(c, layer);
     a.kv = c->kv;
@@ -682,8 +718,8 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         const int64_t base_ctas = (int64_t)c->kv.Hkv * items.n;
         // tensor-core kernel (head_dim 128, at most 16 query heads per KV head): one 8-warp CTA per SM, splits fill
         // the SMs once; the CUDA-core kernel otherwise (and when decode_impl asks for it): four CTAs per SM deep
-        // Prefill rows stay on the f32 CUDA-core kernel unless prefill_impl asks for the tensor-core one
-        // (3.5x faster per 512-row chunk at a 3.5 K prefix, bf16-class error instead of 1e-3)
+        // Prefill rows come here only where launch_split_prefill does not take them, or when prefill_impl asks for the
+        // bf16-class tensor-core kernel
         const bool tc = turbo_mma_supported(c->D, c->G) &&
                         (allow_mma ? c->cfg.decode_impl != GGR_IMPL_SIMT : c->cfg.prefill_impl == GGR_IMPL_MMA);
         const int per_cta_keys = tc ? 2 * kTmWarps * kTmTK : 4 * kTurboGroups;
@@ -998,6 +1034,12 @@ int decode_common(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const f
         return fail(c, GGR_ERR_INVALID, "a KV-sequence shard produces partial states: call ggr_attn_decode_partial");
     if (gate && (partial || gate_head_stride < c->D))
         return fail(c, GGR_ERR_INVALID, "the output gate needs a final output and a head stride of at least head_dim");
+
+    struct HostCall {
+        bool& flag;
+        ~HostCall() { flag = false; }
+    } host_call{c->host_call};
+    c->host_call = ptr_kind == GGR_PTR_HOST;
 
     const size_t qb = (size_t)B * c->q_dim * sizeof(float), kb = (size_t)B * c->kv_dim * sizeof(float);
     // elements from the gate pointer to the end of the last head's row

@@ -104,36 +104,6 @@ __device__ __forceinline__ uint4 turbo_signs8_f16(uint32_t x) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// sign_b . FWHT(sign_a . x) of 128 floats, lane i of the warp holding elements 4 i .. 4 i + 3: the additions of
-// turbo_transform_warp in the same order
-__device__ __forceinline__ void turbo_transform_regs(float (&x)[4], const unsigned char* first, const unsigned char* second,
-                                                     int lane) {
-    const int sh = (lane & 1) * 4;
-    const unsigned fa = first[lane >> 1] >> sh, fb = second[lane >> 1] >> sh;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = (fa >> k) & 1 ? -x[k] : x[k];
-    float a = __fadd_rn(x[0], x[1]), b = __fsub_rn(x[0], x[1]), c = __fadd_rn(x[2], x[3]), d = __fsub_rn(x[2], x[3]);
-    x[0] = __fadd_rn(a, c);
-    x[1] = __fadd_rn(b, d);
-    x[2] = __fsub_rn(a, c);
-    x[3] = __fsub_rn(b, d);
-#pragma unroll
-    for (int w = 1; w < 32; w <<= 1) {
-        const bool upper = lane & w;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float o = __shfl_xor_sync(0xffffffffu, x[k], w);
-            x[k] = upper ? __fsub_rn(o, x[k]) : __fadd_rn(x[k], o);
-        }
-    }
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(128.0f));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        x[k] = __fmul_rn(x[k], scale);
-        x[k] = (fb >> k) & 1 ? -x[k] : x[k];
-    }
-}
-
 inline bool prefill_split_supported(int fmt, int D) {
     return ((fmt == KV_Q8_ROW || fmt == KV_Q8_BLOCK32) && (D == 64 || D == 128)) || (fmt == KV_TURBO && D == 128);
 }
