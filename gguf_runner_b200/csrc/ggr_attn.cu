@@ -237,17 +237,17 @@ void visible_host(const ggr_attn_ctx* c, int layer, int pos, int* vs, int* ve) {
     *ve = e;
 }
 
-// Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, not
-// where copies stand between them (the attribute then only costs host time), and not into a stream capture, where the node in front may be a copy or an event of the caller's.
-bool chain_launches(const ggr_attn_ctx* c) {
-    if (c->timing || c->host_call) return false;
+bool capturing(const ggr_attn_ctx* c) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return st == cudaStreamCaptureStatusNone;
+    return st != cudaStreamCaptureStatusNone;
 }
+// Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, not
+// where copies stand between them (the attribute then only costs host time), and not into a stream capture, where the node in front may be a copy or an event of the caller's.
+bool chain_launches(const ggr_attn_ctx* c) { return !c->timing && !c->host_call && !capturing(c); }
 
 // Brackets one launch with events when kernel timing is on.
 struct LaunchTimer {
@@ -902,7 +902,9 @@ int launch_split_prefill(ggr_attn_ctx* c, int layer, const Items& items, int t_m
     const int slots = c->sm_count * (c->kv.fmt == KV_TURBO ? 1 : 2);
     int limit = std::min(kPsMaxSplits, (t_max + 255) / 256);
     if (c->cfg.max_splits > 0) limit = std::min(limit, c->cfg.max_splits);
-    const int n_split = std::max(1, std::min(limit, slots / (row_tiles * c->kv.Hkv)));
+    int n_split = std::max(1, std::min(limit, slots / (row_tiles * c->kv.Hkv)));
+    const bool fits = (size_t)items.n * c->kv.Hq * n_split * (c->D + 2) <= c->part_cap && (size_t)row_tiles * c->kv.Hkv <= c->counters_cap;
+    if (n_split > 1 && !fits && capturing(c)) n_split = 1;  // (a capture cannot allocate)
     a.n_split = n_split;
     c->last_splits = n_split;
     if (n_split > 1) {
@@ -1224,8 +1226,8 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
                 visible_host(c, layer, std::max(base_pos + i0, base_pos + i0 + n - 2 * kTcBM), &vs1, &ve1);
                 int ns = prefill_tc_splits(n, c->kv.Hq, (std::max(ve, ve1) + kTcBN - 1) / kTcBN - std::min(vs, vs1) / kTcBN, c->sm_count);
                 if (c->cfg.max_splits > 0) ns = std::min(ns, c->cfg.max_splits);
-                if (ns > 1) {
-                    const size_t rows = (size_t)ns * n * c->kv.Hq;
+                const size_t rows = (size_t)ns * n * c->kv.Hq;
+                if (ns > 1 && (rows * (c->D + 2) <= c->part_cap || !capturing(c))) {  // (a capture cannot allocate: unsplit then)
                     int r = ensure(c, &c->d_part, &c->part_cap, rows * (c->D + 2));
                     if (r) return r;
                     a.n_split = ns;
