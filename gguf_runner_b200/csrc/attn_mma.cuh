@@ -320,7 +320,8 @@ inline MmaPlan mma_tma_plan(int D, int warps, int smem_optin) {
     p.ctas_per_sm = (int)((size_t)(smem_optin + 1024) / (p.smem + 4096));
     if (p.ctas_per_sm < 1) p.ctas_per_sm = 1;
     if (p.ctas_per_sm > 4) p.ctas_per_sm = 4;
-    p.min_keys = warps * kTmaTK * 2;
+    // eight warps: down to one tile per warp (2000 keys, 8 KV heads: 7 splits of three rounds -> 16 of one)
+    p.min_keys = warps == kTmaWarps ? warps * kTmaTK - 8 : warps * kTmaTK * 2;
     return p;
 }
 

@@ -246,7 +246,8 @@ bool capturing(const ggr_attn_ctx* c) {
     return st != cudaStreamCaptureStatusNone;
 }
 // Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, not
-// where copies stand between them (the attribute then only costs host time), and not into a stream capture, where the node in front may be a copy or an event of the caller's.
+// where copies stand between them (the attribute then only costs host time), and not into a stream capture,
+// where the node in front may be a copy or an event of the caller's.
 bool chain_launches(const ggr_attn_ctx* c) { return !c->timing && !c->host_call && !capturing(c); }
 
 // Brackets one launch with events when kernel timing is on.
@@ -716,29 +717,29 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             if (rc) return rc;
         }
         const int64_t base_ctas = (int64_t)c->kv.Hkv * items.n;
-        // tensor-core kernel (head_dim 128, at most 16 query heads per KV head): one 8-warp CTA per SM, splits fill
-        // the SMs once; the CUDA-core kernel otherwise (and when decode_impl asks for it): four CTAs per SM deep
+        // tensor-core kernel (head_dim 128, at most 16 query heads per KV head): one 8-warp CTA per SM; the
+        // CUDA-core kernel otherwise (and when decode_impl asks for it): four CTAs per SM deep
         // Prefill rows come here only where launch_split_prefill does not take them, or when prefill_impl asks for the
         // bf16-class tensor-core kernel
         const bool tc = turbo_mma_supported(c->D, c->G) &&
                         (allow_mma ? c->cfg.decode_impl != GGR_IMPL_SIMT : c->cfg.prefill_impl == GGR_IMPL_MMA);
-        const int per_cta_keys = tc ? 2 * kTmWarps * kTmTK : 4 * kTurboGroups;
-        int limit = std::min(64, std::max(1, t_max / per_cta_keys));
+        const int per_cta_keys = tc ? kTmWarps * kTmTK : 4 * kTurboGroups;
+        int limit = std::min(64, std::max(1, tc ? (t_max + per_cta_keys - 1) / per_cta_keys : t_max / per_cta_keys));
         if (c->cfg.max_splits > 0) limit = std::min(limit, c->cfg.max_splits);
         int n_split = (int)std::max<int64_t>(1, ((int64_t)4 * c->sm_count + base_ctas - 1) / base_ctas);
         if (tc) {
-            // the kernel is bound by its own arithmetic (expanding the codes), so what matters is that the last
-            // wave is full: the smallest split count whose CTAs fill at least 95 % of their waves, else the fullest
-            double best_eff = -1.0;
-            n_split = 1;
+            // The kernel is bound by its own arithmetic: a warp takes one 16-key tile after the other, so a CTA costs the
+            // rounds of its eight warps plus a prologue and merge of about four rounds, and the launch as many of these
+            // as it has waves (one CTA per SM). 7777 keys, 4 KV heads: 30 splits of three rounds -> 37 of two.
+            int64_t best = -1;
             for (int n = 1; n <= limit; ++n) {
-                const int64_t ctas = ragged ? (int64_t)c->kv.Hkv * lengths.total(t_max, n) : base_ctas * n, waves = (ctas + c->sm_count - 1) / c->sm_count;
-                const double eff = (double)ctas / (double)(waves * c->sm_count);
-                if (eff > best_eff + 1e-9) {
-                    best_eff = eff;
+                const int64_t ctas = ragged ? (int64_t)c->kv.Hkv * lengths.total(t_max, n) : base_ctas * n;
+                const int64_t waves = (ctas + c->sm_count - 1) / c->sm_count;
+                const int64_t cost = waves * (((t_max + n - 1) / n + per_cta_keys - 1) / per_cta_keys + 4);
+                if (best < 0 || cost < best) {
+                    best = cost;
                     n_split = n;
                 }
-                if (eff >= 0.95) break;
             }
         }
         n_split = std::min(n_split, limit);
