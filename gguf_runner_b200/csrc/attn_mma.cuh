@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int gq = lane >> 2, tq = lane & 3;
-    if (!a.early) decode_begin(a);
+    const bool ahead = decode_ahead(a, item, kvh);
+    if (!ahead) decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     if (prefetched && lane == 0) {
         for (int s = 0; s < NST - 1 && s < my_tiles; ++s) issue(s, s);
     }
-    if (a.early) decode_begin(a);
+    if (ahead) decode_begin(a);
     const float* qsrc = a.q + ((int64_t)item * Hq + (int64_t)kvh * G) * D;
     if (a.fused.enabled) qsrc = fused_rope_prologue(a, item, kvh, seq, pos, owner, smem);
     DECODE_STAMP(1);

@@ -48,6 +48,16 @@ struct PeerExchange {
     int groups_total;
 };
 
+// Loads of cache rows ahead of decode_begin, i.e. before the memory of earlier work in the stream is known to be visible.
+// That is sound where the kernel in front is one of this library's that waited for everything before it and writes no
+// row that is read here; work of the host's own in between (a kernel that writes rows through the addresses of
+// ggr_attn_kv_device_ptrs, a copy, a replayed graph) may do just that.
+//   kAheadKnown   the kernel in front was launched by the same call (projection, fix-ups): no cache rows, nothing between.
+//   kAheadTicket  the decode launch before this one appended to another layer (AttnArgs of that launch are gone, so the
+//                 host says it), and the tickets of its split merge tell whether it is the kernel in front: they are
+//                 nonzero only while it runs, and work of the host's would have started after it.
+constexpr int kAheadNo = 0, kAheadKnown = 1, kAheadTicket = 2;
+
 struct AttnArgs {
     KvView kv;
     Items items;
@@ -63,7 +73,7 @@ struct AttnArgs {
     int shard_count;      // positions held locally
     int stage_bytes;      // bytes of one ring stage of one warp
     int chained;          // launched programmatically behind the kernel in front (launch_chained)
-    int early;            // the kernel in front writes no cache row of this layer: the first tiles may be requested at once
+    int ahead;            // kAhead*: whether the first tiles may be requested before the kernel in front has finished
     int tile_stages;      // ring stages of the CTA-tile kernel (1 or 2)
     int* err;             // raised when a bounded wait runs out (kernels that wait on mbarriers)
     FusedRope fused;
@@ -352,15 +362,24 @@ __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* 
 }
 
 // Decode kernels are launched behind each other (launch_chained): decode_begin waits for the kernel in front. The next
-// one is let in by decode_tail, when every CTA of this grid has reached its merge; its first tiles (AttnArgs::early) then
-// travel while the last CTAs merge. The merge kernel of the fused shard exchange is small and is let in at once: its
-// launch and its wait for the peers' flags overlap this grid's work.
+// one is let in by decode_tail, when every CTA of this grid has reached its merge; its first tiles (decode_ahead) then
+// travel while the last CTAs merge. A launch that is not chained lets nothing in early: the host does not follow the order
+// of those (a captured one runs whenever its graph is replayed). The merge kernel of the fused shard exchange is small and
+// is let in at once: its launch and its wait for the peers' flags overlap this grid's work.
 __device__ __forceinline__ void decode_begin(const AttnArgs& a) {
     if (a.px.enabled) grid_allow_dependents();
     grid_wait();
 }
 __device__ __forceinline__ void decode_tail(const AttnArgs& a) {
-    if (!a.px.enabled) grid_allow_dependents();
+    if (!a.px.enabled && a.chained) grid_allow_dependents();
+}
+
+// Whether this warp may request its first tiles before decode_begin.
+__device__ __forceinline__ bool decode_ahead(const AttnArgs& a, int item, int kvh) {
+    if (a.ahead != kAheadTicket) return a.ahead == kAheadKnown;
+    unsigned arrived;  // relaxed: a count of the launch in flight or the zero it leaves, no data is read on its account
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(arrived) : "l"(a.counters + item * a.kv.Hkv + kvh) : "memory");
+    return __shfl_sync(0xffffffffu, arrived, 0) != 0u;
 }
 
 // Called by the CTA that stored the final states of a (token, kv head) group. When every group of the

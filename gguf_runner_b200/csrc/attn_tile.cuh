@@ -71,7 +71,8 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nst = a.tile_stages;
     DECODE_STAMP(0);
-    if (!a.early) decode_begin(a);
+    const bool ahead = decode_ahead(a, item, kvh);
+    if (!ahead) decode_begin(a);
 
     int seq, pos;
     a.items.get(item, seq, pos);
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
             cp_async_commit();
         }
     }
-    if (a.early) decode_begin(a);
+    if (ahead) decode_begin(a);
     const float* qsrc = a.q + ((int64_t)item * Hq + (int64_t)kvh * G) * D;
     if (a.fused.enabled) qsrc = fused_rope_prologue(a, item, kvh, seq, pos, owner, smem);
     DECODE_STAMP(1);

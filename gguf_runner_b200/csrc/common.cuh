@@ -179,7 +179,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // (launch_chained): the next grid's CTAs take the slots that drain while the last CTAs of the one before it finish, so
 // the launch, the CTA start-up and what does not depend on the predecessor (barriers, tensor memory, weights) cost no
 // time of their own. Every kernel launched that way calls grid_wait() before it touches memory that any earlier work
-// in the stream may write or read; that covers work of other origin too, since the predecessor has waited likewise.
+// in the stream may write or read, whoever enqueued it. The one exception, cache rows that decode kernels request ahead of
+// it, has its rule beside AttnArgs.
 // grid_allow_dependents() comes after grid_wait(): whatever runs ahead of its own grid_wait() can then only meet the one
 // kernel in front of it (the merge kernel of the shard exchange apart, which reads nothing but what flags guard).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

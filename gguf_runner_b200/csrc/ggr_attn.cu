@@ -90,7 +90,7 @@ struct ggr_attn_ctx {
     int* h_err = nullptr;
     int* d_err = nullptr;
     bool host_call = false;  // the decode call in progress has host pointers: copies stand between its kernels
-    int tail_layer = -1;     // layer whose cache rows the last appending launch wrote; -1: unknown
+    int tail_layer = -1;     // layer that the last chained decode launch appended to; -1: none, or an exchange's
     int* d_sched = nullptr;  // work counters of the persistent prefill kernel (rewound by the kernel itself)
     // per-layer pre-attention fixups (device arrays, null = absent) and their f32 scratch rows
     struct LayerFixups {
@@ -346,7 +346,6 @@ int check_layer(ggr_attn_ctx* c, int layer) {
 
 int launch_rope_append(ggr_attn_ctx* c, int layer, const Items& items, int flags, int in_bf16, const void* q,
                        const void* k, const void* v, float* q_out, __nv_bfloat16* q_out_h, float* k_out) {
-    if (flags & RF_APPEND) c->tail_layer = layer;
     if (use_turbo_prep(c) && flags == (RF_ROTATE | RF_WRITE_Q | RF_APPEND)) {
         TurboPrepArgs p{};
         p.rope = rope_params(c, layer);
@@ -667,7 +666,8 @@ struct GateSpec {
 // Attention over the cache for `items` (already rotated q at q_dev).
 // When `raw` is given (decode), q_dev is scratch for the rotated queries: the kernels rotate q and
 // append the k / v row themselves if the fusion scratch fits in shared memory, otherwise the
-// rope/append kernel runs first.
+// rope/append kernel runs first. `front_ours`: the same call has launched the kernel in front (one that waits for the
+// work before it and writes no cache row).
 struct RawDecodeInputs {
     const float* q;
     const float* k;
@@ -676,7 +676,7 @@ struct RawDecodeInputs {
 
 int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, const float* q_dev, float* out_dev,
                      float* partial_dev, bool allow_mma, const RawDecodeInputs* raw = nullptr,
-                     const PeerExchange* px = nullptr, const GateSpec* gate = nullptr) {
+                     const PeerExchange* px = nullptr, const GateSpec* gate = nullptr, bool front_ours = false) {
     AttnArgs a{};
     a.kv = c->kv;
     a.items = items;
@@ -824,10 +824,6 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         }
     }
 
-    // The rows of other layers were complete before the kernel in front began, so the loads of the first tiles overlap
-    // its tail (its split merge, mostly).
-    a.early = a.chained && a.fused.enabled && !px && c->tail_layer >= 0 && c->tail_layer != layer;
-    if (raw) c->tail_layer = px ? -1 : layer;  // (the send kernel of the exchange lets the next one in before it waits itself)
     a.n_split = n_split;
     c->last_splits = n_split;
     if (ragged) lengths.number(t_max, n_split, &a.items);
@@ -853,10 +849,22 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         a.part = c->d_part;
         a.counters = c->d_counters;
     }
+    // Loads ahead of the kernel in front overlap its tail (its split merge, mostly).
+    if (a.chained && a.fused.enabled && !px) {
+        if (front_ours)
+            a.ahead = kAheadKnown;
+        else if (n_split > 1 && c->tail_layer >= 0 && c->tail_layer != layer)
+            a.ahead = kAheadTicket;
+    }
     const dim3 grid = ragged ? dim3(total_splits, c->kv.Hkv, 1) : dim3(n_split, c->kv.Hkv, items.n);
 #ifdef GGR_TC_TRACE
     a.trace = g_tc_trace;
 #endif
+    // (an exchange's send kernel lets the next one in before it waits itself)
+    auto appended = [&]() {
+        if (raw && a.chained) c->tail_layer = px ? -1 : layer;
+        return (int)GGR_OK;
+    };
     if (mma) {
         int rc;
         {
@@ -866,7 +874,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         }
         if (rc != 0) return fail(c, GGR_ERR_CUDA, std::string("mma decode launch: ") + cudaGetErrorString((cudaError_t)rc));
         c->launches++;
-        return GGR_OK;
+        return appended();
     }
     if (tile) {
         int rc;
@@ -876,9 +884,10 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         }
         if (rc != 0) return fail(c, GGR_ERR_CUDA, std::string("tile decode launch: ") + cudaGetErrorString((cudaError_t)rc));
         c->launches++;
-        return GGR_OK;
+        return appended();
     }
-    return launch_simt(c, a, grid, p);
+    const int rc = launch_simt(c, a, grid, p);
+    return rc ? rc : appended();
 }
 
 // Prefill rows of a quantised cache on the tensor cores in 32-bit precision (prefill_split.cuh); `q_dev` holds rotated
@@ -1024,7 +1033,7 @@ int reserve_decode(ggr_attn_ctx* c, int B) {
 
 int decode_common(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const float* q, const float* k,
                   const float* v, float* out, float* partial, int ptr_kind, const float* gate = nullptr,
-                  int gate_head_stride = 0) {
+                  int gate_head_stride = 0, bool front_ours = false) {
     if (!c) return GGR_ERR_INVALID;
     DeviceGuard guard(c->cfg.device);
     int rc = check_layer(c, layer);
@@ -1076,7 +1085,9 @@ int decode_common(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const f
     }
     if ((rc = ensure(c, &c->d_qrot, &c->qrot_cap, (size_t)B * c->q_dim))) return rc;
     int in_bf16 = 0;
+    const void* const before_fixups = dq;
     if ((rc = apply_fixups(c, layer, B, &dq, &dk, &dv, &in_bf16, true))) return rc;
+    front_ours = front_ours || dq != before_fixups;
 
     for (int b0 = 0; b0 < B; b0 += kMaxArgItems) {
         const int n = std::min(kMaxArgItems, B - b0);
@@ -1094,7 +1105,7 @@ int decode_common(ggr_attn_ctx* c, int layer, const int32_t* pos, int B, const f
         float* pc = partial ? dout + (size_t)b0 * c->kv.Hq * (c->D + 2) : nullptr;
         const RawDecodeInputs raw{qc, kc, vc};
         GateSpec gs{dgate ? dgate + (size_t)b0 * c->kv.Hq * gate_head_stride : nullptr, gate_head_stride, 0};
-        rc = launch_attention(c, layer, it, t_max, qr, oc, pc, true, &raw, nullptr, &gs);
+        rc = launch_attention(c, layer, it, t_max, qr, oc, pc, true, &raw, nullptr, &gs, front_ours && b0 == 0);
         if (rc) return rc;
     }
     if (ptr_kind == GGR_PTR_HOST) {
@@ -2791,7 +2802,7 @@ extern "C" int ggr_attn_layer_decode(ggr_attn_ctx* c, int32_t layer, const int32
     } else {
         if ((rc = matmul_qkv_device(c, wq, wk, wv, dx, B, dq, dk, dv))) return rc;
     }
-    if ((rc = decode_common(c, layer, pos, B, dq, dk, dv, c->d_patt, nullptr, GGR_PTR_DEVICE))) return rc;
+    if ((rc = decode_common(c, layer, pos, B, dq, dk, dv, c->d_patt, nullptr, GGR_PTR_DEVICE, nullptr, 0, true))) return rc;
     if ((rc = matmul_device(c, wo, c->d_patt, B, dout, nullptr, dim_out, 1))) return rc;
     if (ptr_kind == GGR_PTR_HOST) {
         const size_t out_bytes = (size_t)B * dim_out * sizeof(float);

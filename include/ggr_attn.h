@@ -389,7 +389,12 @@ int ggr_attn_kernel_time(ggr_attn_ctx* ctx, int32_t kind, double* total_ms, int6
 /* Device addresses of the cache arrays (layout: [sequence][layer][position -
  * shard_pos_begin][kv_dim] in the configured format; scales are null unless
  * the format is q8) and the byte size of one of the K / V arrays. For hosts
- * that keep K/V producers on the device, and for synthetic cache fills. */
+ * that keep K/V producers on the device, and for synthetic cache fills.
+ * Kernels, copies and graphs of the host's that write rows are ordered by the stream like any other work. Decode launches
+ * overlap their first loads with the end of the decode launch in front of them, and only there: work in between ends the
+ * overlap. (A kernel that the host itself launches programmatically, that lets its own dependents in with
+ * griddepcontrol.launch_dependents before it has waited for the work in front of it, and that writes cache rows, would not
+ * be such an end: such a writer has to wait first.) */
 int ggr_attn_kv_device_ptrs(ggr_attn_ctx* ctx, void** k, void** v, float** k_scale, float** v_scale,
                             uint64_t* array_bytes);
 
