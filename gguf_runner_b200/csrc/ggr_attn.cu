@@ -53,6 +53,12 @@ struct ggr_attn_ctx {
     size_t part_cap = 0;
     unsigned* d_counters = nullptr;
     size_t counters_cap = 0;
+    // the same of prefill launches, apart from the decode scratch: that one is reserved at create time, captured decode
+    // launches keep its address, and its size bounds their splits
+    float* d_part_p = nullptr;
+    size_t part_p_cap = 0;
+    unsigned* d_counters_p = nullptr;
+    size_t counters_p_cap = 0;
     // staging for host-pointer calls
     unsigned char* d_stage[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // q, k, v, out, gate
     size_t stage_cap[5] = {0, 0, 0, 0, 0};
@@ -656,6 +662,21 @@ int plan_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, in
     return n;
 }
 
+// Partial-state floats and tickets (zero between launches) of a split launch; nothing grows within a reservation.
+int split_scratch(ggr_attn_ctx* c, bool prefill, size_t floats, size_t tickets, float** part, unsigned** counters) {
+    float** p = prefill ? &c->d_part_p : &c->d_part;
+    unsigned** t = prefill ? &c->d_counters_p : &c->d_counters;
+    size_t* t_cap = prefill ? &c->counters_p_cap : &c->counters_cap;
+    int rc = ensure(c, p, prefill ? &c->part_p_cap : &c->part_cap, floats);
+    if (rc) return rc;
+    const size_t before = *t_cap;
+    if ((rc = ensure(c, t, t_cap, tickets))) return rc;
+    if (*t_cap != before) CUDA_TRY(c, cudaMemsetAsync(*t, 0, *t_cap * sizeof(unsigned), c->stream));
+    *part = *p;
+    *counters = *t;
+    return GGR_OK;
+}
+
 // Output gate of a call (src/engine/runtime/inference.rs:3509-3519); p == nullptr = none.
 struct GateSpec {
     const void* p;
@@ -750,15 +771,9 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         a.n_split = n_split;
         c->last_splits = n_split;
         if (n_split > 1) {
-            int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)total * c->kv.Hq * (c->D + 2));
+            int rc = split_scratch(c, items.mode == 1, (size_t)total * c->kv.Hq * (c->D + 2), (size_t)items.n * c->kv.Hkv, &a.part,
+                                   &a.counters);
             if (rc) return rc;
-            const size_t before = c->counters_cap;
-            rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)items.n * c->kv.Hkv);
-            if (rc) return rc;
-            if (c->counters_cap != before)
-                CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, c->counters_cap * sizeof(unsigned), c->stream));
-            a.part = c->d_part;
-            a.counters = c->d_counters;
         }
         int e;
         if (tc) {
@@ -839,15 +854,9 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         smem = p.smem = (size_t)a.fused.smem_off + fb;
     }
     if (n_split > 1) {
-        int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)total_splits * c->kv.Hq * (c->D + 2));
+        int rc = split_scratch(c, items.mode == 1, (size_t)total_splits * c->kv.Hq * (c->D + 2), (size_t)items.n * c->kv.Hkv, &a.part,
+                               &a.counters);
         if (rc) return rc;
-        const size_t before = c->counters_cap;
-        rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)items.n * c->kv.Hkv);
-        if (rc) return rc;
-        if (c->counters_cap != before)
-            CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, c->counters_cap * sizeof(unsigned), c->stream));
-        a.part = c->d_part;
-        a.counters = c->d_counters;
     }
     // Loads ahead of the kernel in front overlap its tail (its split merge, mostly).
     if (a.chained && a.fused.enabled && !px) {
@@ -890,6 +899,30 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     return rc ? rc : appended();
 }
 
+// CTAs of prefill_split_kernel that run at a time
+int split_prefill_slots(const ggr_attn_ctx* c) { return c->sm_count * (c->kv.fmt == KV_TURBO ? 1 : 2); }
+
+bool use_prefill_tc(const ggr_attn_ctx* c) {
+    return c->have_tmaps && prefill_tc_usable(c->cfg.prefill_impl, c->kv.fmt, c->D, c->G);
+}
+bool use_split_prefill(const ggr_attn_ctx* c) {
+    return c->cfg.prefill_impl == GGR_IMPL_AUTO && prefill_split_supported(c->kv.fmt, c->D);
+}
+
+// Scratch for the largest split launch of the tensor-core prefill kernels: both split only as far as their CTAs run at a
+// time, i.e. 256 rows per SM (bf16 caches) or 64 per slot (quantised ones); 20 MB at head_dim 128. Reserved at create time
+// so that a chunk splits the same way under stream capture, and a captured one keeps its address. A device too full for
+// it is no error: launches that find no scratch do not split.
+int reserve_prefill(ggr_attn_ctx* c) {
+    if (c->cfg.max_splits == 1 || c->cfg.shard_mode != GGR_SHARD_NONE) return GGR_OK;
+    const size_t slots = split_prefill_slots(c);
+    float* part;
+    unsigned* counters;
+    if (use_prefill_tc(c)) return split_scratch(c, true, (size_t)c->sm_count * 2 * kTcBM * (c->D + 2), 1, &part, &counters);
+    if (use_split_prefill(c)) return split_scratch(c, true, slots * kPsRows * (c->D + 2), slots, &part, &counters);
+    return GGR_OK;
+}
+
 // Prefill rows of a quantised cache on the tensor cores in 32-bit precision (prefill_split.cuh); `q_dev` holds rotated
 // queries, the rows are appended already.
 int launch_split_prefill(ggr_attn_ctx* c, int layer, const Items& items, int t_max, const float* q_dev, float* out_dev,
@@ -909,24 +942,17 @@ int launch_split_prefill(ggr_attn_ctx* c, int layer, const Items& items, int t_m
         a.gate_head_stride = gate.head_stride;
     }
     const int row_tiles = (items.n * c->G + kPsRows - 1) / kPsRows;
-    const int slots = c->sm_count * (c->kv.fmt == KV_TURBO ? 1 : 2);
+    const int slots = split_prefill_slots(c);
     int limit = std::min(kPsMaxSplits, (t_max + 255) / 256);
     if (c->cfg.max_splits > 0) limit = std::min(limit, c->cfg.max_splits);
     int n_split = std::max(1, std::min(limit, slots / (row_tiles * c->kv.Hkv)));
-    const bool fits = (size_t)items.n * c->kv.Hq * n_split * (c->D + 2) <= c->part_cap && (size_t)row_tiles * c->kv.Hkv <= c->counters_cap;
-    if (n_split > 1 && !fits && capturing(c)) n_split = 1;  // (a capture cannot allocate)
+    const size_t part_floats = (size_t)items.n * c->kv.Hq * n_split * (c->D + 2), tickets = (size_t)row_tiles * c->kv.Hkv;
+    if (part_floats > c->part_p_cap || tickets > c->counters_p_cap) n_split = 1;
     a.n_split = n_split;
     c->last_splits = n_split;
     if (n_split > 1) {
-        int rc = ensure(c, &c->d_part, &c->part_cap, (size_t)items.n * c->kv.Hq * n_split * (c->D + 2));
-        if (rc) return rc;
-        const size_t before = c->counters_cap;
-        rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)row_tiles * c->kv.Hkv);
-        if (rc) return rc;
-        if (c->counters_cap != before)
-            CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, c->counters_cap * sizeof(unsigned), c->stream));
-        a.part = c->d_part;
-        a.counters = c->d_counters;
+        a.part = c->d_part_p;
+        a.counters = c->d_counters_p;
     }
     {
         LaunchTimer t(c, 0);
@@ -1015,11 +1041,9 @@ int reserve_decode(ggr_attn_ctx* c, int B) {
     const int chunk = std::min(B, kMaxArgItems);
     if (splits > 1 || ragged_rows > 0) {
         const size_t rows = std::max(chunk * splits, ragged_rows);
-        if ((rc = ensure(c, &c->d_part, &c->part_cap, rows * c->kv.Hq * (c->D + 2)))) return rc;
-        const size_t before = c->counters_cap;
-        if ((rc = ensure(c, &c->d_counters, &c->counters_cap, (size_t)chunk * c->kv.Hkv))) return rc;
-        if (c->counters_cap != before)
-            CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, c->counters_cap * sizeof(unsigned), c->stream));
+        float* part;
+        unsigned* counters;
+        if ((rc = split_scratch(c, false, rows * c->kv.Hq * (c->D + 2), (size_t)chunk * c->kv.Hkv, &part, &counters))) return rc;
     }
     // host-pointer calls: q | k | v | gate inbound (a packed gate spans up to 2 * q_dim per token), out or partial outbound
     const size_t in_bytes = ((size_t)B * (c->q_dim + 2 * c->kv_dim) + (size_t)B * 2 * c->q_dim) * sizeof(float);
@@ -1176,7 +1200,7 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
     }
 
     const bool wide = c->have_tmaps64 && c->cfg.prefill_impl != GGR_IMPL_SIMT;
-    const bool tc = wide || (c->have_tmaps && prefill_tc_usable(c->cfg.prefill_impl, c->kv.fmt, c->D, c->G));
+    const bool tc = wide || use_prefill_tc(c);
     if (c->cfg.prefill_impl == GGR_IMPL_TCGEN05 && !tc)
         return fail(c, GGR_ERR_UNSUPPORTED, "the tensor-core prefill kernels need a bf16 cache and head_dim 64, 128 or 256");
     if ((rc = ensure(c, &c->d_qrot, &c->qrot_cap, tc ? (size_t)1 : (size_t)m * c->q_dim))) return rc;
@@ -1239,12 +1263,10 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
                 int ns = prefill_tc_splits(n, c->kv.Hq, (std::max(ve, ve1) + kTcBN - 1) / kTcBN - std::min(vs, vs1) / kTcBN, c->sm_count);
                 if (c->cfg.max_splits > 0) ns = std::min(ns, c->cfg.max_splits);
                 const size_t rows = (size_t)ns * n * c->kv.Hq;
-                if (ns > 1 && (rows * (c->D + 2) <= c->part_cap || !capturing(c))) {  // (a capture cannot allocate: unsplit then)
-                    int r = ensure(c, &c->d_part, &c->part_cap, rows * (c->D + 2));
-                    if (r) return r;
+                if (ns > 1 && rows * (c->D + 2) <= c->part_p_cap) {
                     a.n_split = ns;
-                    a.part = c->d_part;
-                    a.ml = reinterpret_cast<float2*>(c->d_part + rows * c->D);
+                    a.part = c->d_part_p;
+                    a.ml = reinterpret_cast<float2*>(a.part + rows * c->D);
                 }
             }
 #ifdef GGR_TC_TRACE
@@ -1290,7 +1312,7 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
             }
             const float* qr = c->d_qrot + (size_t)j0 * c->q_dim;
             float* o = dout + (size_t)j0 * c->q_dim;
-            int r = c->cfg.prefill_impl == GGR_IMPL_AUTO && prefill_split_supported(c->kv.fmt, c->D)
+            int r = use_split_prefill(c)
                         ? launch_split_prefill(c, layer, it, t_max, qr, o, gs)
                         : launch_attention(c, layer, it, t_max, qr, o, nullptr, false, nullptr, nullptr, &gs);
             if (r) return r;
@@ -1554,6 +1576,11 @@ int ggr_attn_create(const ggr_attn_config* cfg, ggr_attn_ctx** out) {
     c->x_wait_ns = cfg->exchange_wait_us > 0 ? (unsigned long long)cfg->exchange_wait_us * 1000ull : 1000000000ull;
     // decode scratch for max_batch sequences, so that the token loop never allocates (see ggr_attn_reserve)
     if (int rr = reserve_decode(c, std::min(cfg->max_batch, kMaxArgItems))) return cleanup(rr, c->err);
+    if (int rr = reserve_prefill(c)) {
+        if (rr != GGR_ERR_ALLOC) return cleanup(rr, c->err);
+        cudaGetLastError();
+        c->err.clear();
+    }
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(GGR_ERR_CUDA, "device initialisation failed");
     g_create_err.clear();
     *out = c;
@@ -1581,6 +1608,8 @@ void ggr_attn_destroy(ggr_attn_ctx* c) {
     cudaFree(c->d_qrot);
     cudaFree(c->d_qrot_h);
     cudaFree(c->d_part);
+    cudaFree(c->d_part_p);
+    cudaFree(c->d_counters_p);
     cudaFree(c->d_counters);
     for (auto* p : c->d_stage) cudaFree(p);
     cudaFree(c->d_gate_f32);
