@@ -95,6 +95,8 @@ struct ggr_attn_ctx {
     // error word the kernels raise when a bounded wait runs out (mapped pinned host memory)
     int* h_err = nullptr;
     int* d_err = nullptr;
+    bool captured = false;         // launches of this context have been captured into a graph
+    std::vector<void*> retired;    // scratch that was outgrown after that, kept for the graphs
     bool host_call = false;  // the decode call in progress has host pointers: copies stand between its kernels
     int tail_layer = -1;     // layer that the last chained decode launch appended to; -1: none, or an exchange's
     int* d_sched = nullptr;  // work counters of the persistent prefill kernel (rewound by the kernel itself)
@@ -181,10 +183,16 @@ int ensure(ggr_attn_ctx* c, T** ptr, size_t* cap, size_t need_elems) {
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (c->copy_in) CUDA_TRY(c, cudaStreamSynchronize(c->copy_in));
     if (c->copy_out) CUDA_TRY(c, cudaStreamSynchronize(c->copy_out));
-    if (*ptr) cudaFree(*ptr);
+    size_t want = std::max(need_elems, (size_t)256);
+    if (*ptr && c->captured) {
+        // a graph may still write the old buffer; doubling keeps what is kept for graphs below the buffer in use
+        c->retired.push_back(*ptr);
+        want = std::max(want, 2 * *cap);
+    } else if (*ptr) {
+        cudaFree(*ptr);
+    }
     *ptr = nullptr;
     *cap = 0;
-    size_t want = std::max(need_elems, (size_t)256);
     cudaError_t e = cudaMalloc((void**)ptr, want * sizeof(T));
     if (e != cudaSuccess) return fail(c, GGR_ERR_ALLOC, std::string("scratch allocation failed: ") + cudaGetErrorString(e));
     *cap = want;
@@ -243,18 +251,19 @@ void visible_host(const ggr_attn_ctx* c, int layer, int pos, int* vs, int* ve) {
     *ve = e;
 }
 
-bool capturing(const ggr_attn_ctx* c) {
+bool capturing(ggr_attn_ctx* c) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
         cudaGetLastError();
         return true;
     }
+    if (st != cudaStreamCaptureStatusNone) c->captured = true;
     return st != cudaStreamCaptureStatusNone;
 }
 // Whether launches are programmatic (launch_chained): not while per-kernel event pairs are recorded between them, not
 // where copies stand between them (the attribute then only costs host time), and not into a stream capture,
 // where the node in front may be a copy or an event of the caller's.
-bool chain_launches(const ggr_attn_ctx* c) { return !c->timing && !c->host_call && !capturing(c); }
+bool chain_launches(ggr_attn_ctx* c) { return !c->host_call && !capturing(c) && !c->timing; }
 
 // Brackets one launch with events when kernel timing is on.
 struct LaunchTimer {
@@ -1608,6 +1617,7 @@ void ggr_attn_destroy(ggr_attn_ctx* c) {
     cudaFree(c->d_qrot);
     cudaFree(c->d_qrot_h);
     cudaFree(c->d_part);
+    for (void* p : c->retired) cudaFree(p);
     cudaFree(c->d_part_p);
     cudaFree(c->d_counters_p);
     cudaFree(c->d_counters);
