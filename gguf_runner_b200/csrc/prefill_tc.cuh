@@ -126,12 +126,16 @@ struct TcItem {
 };
 
 // Items are numbered longest first: late query rows see the most keys.
+template <bool SPLIT>
 __device__ __forceinline__ TcItem tc_item(const PrefillTcArgs& a, int r) {
     TcItem it;
     const int Hq = a.kv.Hq;
     const int n_pairs = (a.m + 2 * kTcBM - 1) / (2 * kTcBM);
-    it.split = r % a.n_split;
-    r /= a.n_split;
+    it.split = 0;
+    if constexpr (SPLIT) {
+        it.split = r % a.n_split;
+        r /= a.n_split;
+    }
     const int pair = n_pairs - 1 - r / Hq;
     it.h = r % Hq;
     it.kvh = it.h / a.kv.G;
@@ -151,7 +155,7 @@ __device__ __forceinline__ TcItem tc_item(const PrefillTcArgs& a, int r) {
         lo_t[t] = min(vs0, vs1) / kTcBN;
         hi_t[t] = (max(ve0, ve1) + kTcBN - 1) / kTcBN;
     }
-    if (a.n_split > 1) {
+    if constexpr (SPLIT) {
         const int lo = hi_t[1] > lo_t[1] ? min(lo_t[0], lo_t[1]) : lo_t[0], hi = max(hi_t[0], hi_t[1]);
         const int chunk = (hi - lo + a.n_split - 1) / a.n_split, s_lo = lo + it.split * chunk, s_hi = min(hi, s_lo + chunk);
 #pragma unroll
@@ -171,7 +175,9 @@ __device__ __forceinline__ TcItem tc_item(const PrefillTcArgs& a, int r) {
     return it;
 }
 
-template <int D>
+// SPLIT: key splits, an instantiation of its own. A whole prompt has no use for the divisions of tc_item in four roles and
+// the choices of the epilogue (32/8 heads of 128, 4096 rows, rope included: 174 -> 170 us per layer without them).
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, PrefillTcArgs a) {
@@ -260,7 +266,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                 itemp[slot] = r;
                 mbar_arrive(item_full(slot));
                 if (r < 0) break;
-                const TcItem w = tc_item(a, r);
+                const TcItem w = tc_item<SPLIT>(a, r);
                 const bool act0 = w.hi0 > w.lo0, act1 = w.hi1 > w.lo1;
                 if (!mbar_wait(q_empty, (it & 1) ^ 1, abortp)) break;
                 mbar_expect_tx(q_full, ((act0 ? 1 : 0) + (act1 ? 1 : 0)) * TILE_BYTES);
@@ -335,7 +341,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             const int r = __shfl_sync(0xffffffffu, itemp[slot], 0);
             if (lane == 0) mbar_arrive(item_empty(slot));
             if (r < 0) break;
-            const TcItem w = tc_item(a, r);
+            const TcItem w = tc_item<SPLIT>(a, r);
             const int lo = w.lo, hi = w.hi;
             // Every item moves o_free and o_final of both tiles on by one phase. A tile without visible keys
             // does that here; an active tile waits for o_free right before its first P V overwrites O_t.
@@ -446,7 +452,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(item_empty(slot));
             if (r < 0) break;
-            const TcItem w = tc_item(a, r);
+            const TcItem w = tc_item<SPLIT>(a, r);
             const int lo_t = w.lo_of(t), hi_t = w.hi_of(t), n_t = hi_t - lo_t;
 #ifdef GGR_TC_TRACE
             const int lo = w.lo;
@@ -572,7 +578,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             TRACE_ADD(ts_ofin);
             fence_after_sync();
             float* orow0 = a.out;
-            if (a.n_split > 1) {
+            if constexpr (SPLIT) {
                 orow0 = a.part + (int64_t)w.split * a.m * Hq * D;
                 if (valid) a.ml[((int64_t)w.split * a.m + qi) * Hq + w.h] = make_float2(m_used, l);
             }
@@ -582,9 +588,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                 // warp hit different banks; the warp then reads the area back four rows at a time and stores
                 // whole 128-byte lines. One thread per row storing 16-byte pieces 16 KB apart cost a cache-line
                 // wavefront per lane and instruction, 3-4 us per item during which the tile's pipeline stood still.
-                const float inv = a.n_split > 1 ? 1.0f : (l > 0.0f ? 1.0f / l : 0.0f);
+                const float inv = SPLIT ? 1.0f : (l > 0.0f ? 1.0f / l : 0.0f);
                 const void* grow = nullptr;
-                if (a.gate && valid && a.n_split == 1)
+                if (!SPLIT && a.gate && valid)
                     grow = static_cast<const unsigned char*>(a.gate) +
                            ((int64_t)qi * Hq + w.h) * a.gate_head_stride * (a.gate_bf16 ? 2 : 4);
                 const uint32_t stage = sOut + (uint32_t)warp * 4096u;
@@ -711,14 +717,14 @@ inline bool prefill_tc_usable(int impl, int fmt, int D, int /*G*/) {
 
 inline size_t prefill_tc_smem(int D) { return (size_t)6 * (D / 64) * 128 * 128 + 8 * 4096 + 1024; }
 
-template <int D>
+template <int D, bool SPLIT>
 inline int launch_prefill_tc_inst(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                                   const PrefillTcArgs& a, int device, int sm_count, cudaStream_t stream,
                                   std::string* msg) {
     static KernelSmemSetup setup;
     const size_t smem = prefill_tc_smem(D);
     {
-        const cudaError_t e = setup.ensure(prefill_tc_kernel<D>, device, 0, (int)smem);
+        const cudaError_t e = setup.ensure(prefill_tc_kernel<D, SPLIT>, device, 0, (int)smem);
         if (e != cudaSuccess) {
             *msg = std::string("prefill kernel attribute: ") + cudaGetErrorString(e);
             return 2;
@@ -744,16 +750,16 @@ inline int launch_prefill_tc_inst(const CUtensorMap& tq, const CUtensorMap& tk, 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         lc.attrs = attr;
         lc.numAttrs = 1;
-        e = cudaLaunchKernelEx(&lc, prefill_tc_kernel<D>, tq, tk, tv, args);
+        e = cudaLaunchKernelEx(&lc, prefill_tc_kernel<D, SPLIT>, tq, tk, tv, args);
     } else {
-        prefill_tc_kernel<D><<<grid, kTcThreads, smem, stream>>>(tq, tk, tv, args);
+        prefill_tc_kernel<D, SPLIT><<<grid, kTcThreads, smem, stream>>>(tq, tk, tv, args);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
         *msg = std::string("prefill kernel launch: ") + cudaGetErrorString(e);
         return 2;
     }
-    if (args.n_split > 1) {
+    if constexpr (SPLIT) {
         const int64_t threads = (int64_t)a.m * a.kv.Hq * (D / 4);
         e = launch_chained(args.dependent != 0, prefill_merge_kernel<D>, dim3((unsigned)((threads + 255) / 256)), 256, 0, stream, args);
         if (e != cudaSuccess) {
@@ -773,8 +779,10 @@ inline int launch_prefill_tc(const PrefillTcArgs& a, const CUtensorMap& tk, cons
         return 2;
     }
     switch (a.kv.D) {
-        case 64: return launch_prefill_tc_inst<64>(tq, tk, tv, a, device, sm_count, stream, msg);
-        case 128: return launch_prefill_tc_inst<128>(tq, tk, tv, a, device, sm_count, stream, msg);
+        case 64: return a.n_split > 1 ? launch_prefill_tc_inst<64, true>(tq, tk, tv, a, device, sm_count, stream, msg)
+                                      : launch_prefill_tc_inst<64, false>(tq, tk, tv, a, device, sm_count, stream, msg);
+        case 128: return a.n_split > 1 ? launch_prefill_tc_inst<128, true>(tq, tk, tv, a, device, sm_count, stream, msg)
+                                       : launch_prefill_tc_inst<128, false>(tq, tk, tv, a, device, sm_count, stream, msg);
         default: *msg = "no tensor-core prefill kernel for this head_dim"; return 5;
     }
 }
