@@ -1290,6 +1290,12 @@ int prefill_common(ggr_attn_ctx* c, int layer, int seq, int base_pos, int m, con
             }
             if (r) return fail(c, r, msg);
             c->launches++;
+            c->last_splits = a.n_split;
+            if (a.n_split > 1) {
+                LaunchTimer t(c, 2);
+                CUDA_TRY(c, launch_prefill_merge(a, c->stream));
+                c->launches++;
+            }
             return GGR_OK;
         }
         const int max_items = 65535;

@@ -759,15 +759,14 @@ inline int launch_prefill_tc_inst(const CUtensorMap& tq, const CUtensorMap& tk, 
         *msg = std::string("prefill kernel launch: ") + cudaGetErrorString(e);
         return 2;
     }
-    if constexpr (SPLIT) {
-        const int64_t threads = (int64_t)a.m * a.kv.Hq * (D / 4);
-        e = launch_chained(args.dependent != 0, prefill_merge_kernel<D>, dim3((unsigned)((threads + 255) / 256)), 256, 0, stream, args);
-        if (e != cudaSuccess) {
-            *msg = std::string("prefill merge launch: ") + cudaGetErrorString(e);
-            return 2;
-        }
-    }
     return 0;
+}
+
+// the merge behind a launch with key splits
+inline cudaError_t launch_prefill_merge(const PrefillTcArgs& a, cudaStream_t stream) {
+    const int64_t threads = (int64_t)a.m * a.kv.Hq * (a.kv.D / 4);
+    return launch_chained(a.dependent != 0, a.kv.D == 64 ? prefill_merge_kernel<64> : prefill_merge_kernel<128>,
+                          dim3((unsigned)((threads + 255) / 256)), 256, 0, stream, a);
 }
 
 // tk / tv describe the whole K and V cache arrays as [rows][kv_dim].

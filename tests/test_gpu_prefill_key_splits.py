@@ -26,7 +26,26 @@ def test_splits_match_the_unsplit_launch(head_dim, heads, kv_heads, window):
         assert np.max(np.abs(got - want)) <= 1e-2, m
         got, want = (c.prefill_gated(0, pos, q, k, v, gate) for c in ctxs)
         assert np.max(np.abs(got - want)) <= 1e-2, m
+        if pos:  # at least 12 visible key tiles and at most 64 query tiles x heads: two splits and more
+            assert ctxs[0].last_split_count > 1 and ctxs[1].last_split_count == 1, m
         pos += m
+
+
+def test_merge_launches_are_counted_and_timed():
+    import torch
+    counts = []
+    for max_splits in (0, 1):
+        ctx = g.AttnContext(AttnConfig(n_layers=1, n_heads=8, n_kv_heads=2, head_dim=128, seq_len=3000, rope_theta=1e6,
+                                       rope_style=ROPE_NEOX, kv_format=KV_BF16, max_splits=max_splits))
+        rows = [torch.randn(40, d, device="cuda") for d in (ctx.config.q_dim, ctx.config.kv_dim, ctx.config.kv_dim)]
+        before = ctx.launch_count
+        ctx.prefill(0, 2900, *rows)
+        ctx.set_kernel_timing(True)
+        after = ctx.launch_count
+        ctx.prefill(0, 2900, *rows)
+        counts.append((after - before, ctx.kernel_time(0)[1], ctx.kernel_time(1)[1], ctx.kernel_time(2)[1]))
+        ctx.close()
+    assert counts == [(3, 1, 1, 1), (2, 1, 1, 0)]
 
 
 def test_image_blocks_with_splits():
@@ -40,3 +59,4 @@ def test_image_blocks_with_splits():
         rows = [rng.standard_normal((m, d)).astype(np.float32) for d in (cfg.q_dim, cfg.kv_dim, cfg.kv_dim)]
         got, want = (getattr(c, call)(0, pos, *rows) for c in ctxs)
         assert np.max(np.abs(got - want)) <= 1e-2
+        assert ctxs[0].last_split_count > 1 and ctxs[1].last_split_count == 1
