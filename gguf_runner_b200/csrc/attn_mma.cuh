@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_mma_decode_kernel(AttnArg
     constexpr int NT = D / 8;    // n-tiles of P.V
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attn_mma_decode_kernel(AttnArg
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -325,10 +325,13 @@ inline MmaPlan mma_tma_plan(int D, int warps, int smem_optin) {
     return p;
 }
 
+template <int W>
+using TmaArgs = std::conditional_t<W == kTmaWarps, AttnArgs, RaggedAttnArgs>;
+
 template <int D, int W>
 __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                              const __grid_constant__ CUtensorMap tmV,
-                                                                             AttnArgs a) {
+                                                                             TmaArgs<W> a) {
     using namespace tc;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t s_full[W][kTmaNST];
@@ -343,8 +346,8 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     constexpr int NST = kTmaNST;
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -566,7 +569,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
 }
 
 template <int D, int W>
-inline int launch_mma_tma_inst(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid, size_t smem,
+inline int launch_mma_tma_inst(const CUtensorMap& tk, const CUtensorMap& tv, const TmaArgs<W>& a, dim3 grid, size_t smem,
                                int smem_optin, int device, cudaStream_t stream) {
     static KernelSmemSetup setup;
     const cudaError_t se = setup.ensure(attn_mma_tma_decode_kernel<D, W>, device, smem_optin);
@@ -574,14 +577,15 @@ inline int launch_mma_tma_inst(const CUtensorMap& tk, const CUtensorMap& tv, con
     return (int)launch_chained(a.chained, attn_mma_tma_decode_kernel<D, W>, grid, W * 32, smem, stream, tk, tv, a);
 }
 
-// tk / tv: tensor maps over the whole K and V arrays with a box of 64 columns x 16 rows
-inline int launch_mma_tma_decode(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, int warps, dim3 grid,
-                                 size_t smem, int smem_optin, int device, cudaStream_t stream) {
+// tk / tv: tensor maps over the whole K and V arrays with a box of 64 columns x 16 rows. Args: AttnArgs (eight warps) or
+// RaggedAttnArgs (four).
+template <typename Args>
+inline int launch_mma_tma_decode(const CUtensorMap& tk, const CUtensorMap& tv, const Args& a, dim3 grid, size_t smem,
+                                 int smem_optin, int device, cudaStream_t stream) {
+    constexpr int W = std::is_same_v<Args, AttnArgs> ? kTmaWarps : kTmaWarpsRagged;
     switch (a.kv.D) {
-        case 64: return warps == kTmaWarps ? launch_mma_tma_inst<64, kTmaWarps>(tk, tv, a, grid, smem, smem_optin, device, stream)
-                                           : launch_mma_tma_inst<64, kTmaWarpsRagged>(tk, tv, a, grid, smem, smem_optin, device, stream);
-        case 128: return warps == kTmaWarps ? launch_mma_tma_inst<128, kTmaWarps>(tk, tv, a, grid, smem, smem_optin, device, stream)
-                                            : launch_mma_tma_inst<128, kTmaWarpsRagged>(tk, tv, a, grid, smem, smem_optin, device, stream);
+        case 64: return launch_mma_tma_inst<64, W>(tk, tv, a, grid, smem, smem_optin, device, stream);
+        case 128: return launch_mma_tma_inst<128, W>(tk, tv, a, grid, smem, smem_optin, device, stream);
         default: return (int)cudaErrorNotSupported;
     }
 }

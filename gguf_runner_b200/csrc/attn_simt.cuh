@@ -87,29 +87,44 @@ struct AttnArgs {
 #endif
 };
 
-// Which item and which of its n splits a CTA works on; state of (head h, split s): row first + h * n + s of a.part.
-struct SplitPos {
-    int item, split, n;
-    int64_t first;
+// Decode of sequences of different lengths: item i is split split0[i + 1] - split0[i] ways, and the splits of all items are
+// numbered one after the other in blockIdx.x. Kernels that take such launches have an instantiation for them, and the
+// other one reads its position from the block indices wherever it needs it: with the position of either kind held in
+// registers across the kernel (the CTA-tile kernel has none to spare) and the table among the parameters of every launch, a
+// host-pointer decode of 1501 keys (q8 cache, 32/8 heads) takes 44.0 us per layer against 43.5, one of f32 rows, 700 keys,
+// 41.1 against 40.4.
+struct RaggedAttnArgs : AttnArgs {
+    unsigned short split0[kMaxArgItems + 1];
 };
-__device__ __forceinline__ SplitPos split_pos(const AttnArgs& a) {
-    SplitPos sp;
-    if (a.items.ragged) {
-        int lo = 0, hi = a.items.n - 1;  // the last item that starts at or before this split
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (a.items.split0[mid] <= blockIdx.x)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        lo = __shfl_sync(0xffffffffu, lo, 0);  // (tells the compiler that the result is warp-uniform)
-        const int s0 = a.items.split0[lo];
-        sp = SplitPos{lo, (int)blockIdx.x - s0, a.items.split0[lo + 1] - s0, (int64_t)s0 * a.kv.Hq};
-    } else {
-        sp = SplitPos{(int)blockIdx.z, (int)blockIdx.x, a.n_split, (int64_t)blockIdx.z * a.kv.Hq * a.n_split};
+
+// Which item and which of its n() splits a CTA works on, and the row of a.part that holds the state of (head, split).
+struct UniformPos {
+    const AttnArgs& a;
+    __device__ __forceinline__ int item() const { return blockIdx.z; }
+    __device__ __forceinline__ int split() const { return blockIdx.x; }
+    __device__ __forceinline__ int n() const { return a.n_split; }
+    __device__ __forceinline__ int64_t row(int h, int s) const { return ((int64_t)blockIdx.z * a.kv.Hq + h) * a.n_split + s; }
+};
+struct RaggedPos {
+    const AttnArgs& a;
+    int item_, s0, n_;
+    __device__ __forceinline__ int item() const { return item_; }
+    __device__ __forceinline__ int split() const { return (int)blockIdx.x - s0; }
+    __device__ __forceinline__ int n() const { return n_; }
+    __device__ __forceinline__ int64_t row(int h, int s) const { return (int64_t)s0 * a.kv.Hq + (int64_t)h * n_ + s; }
+};
+__device__ __forceinline__ UniformPos split_pos(const AttnArgs& a) { return UniformPos{a}; }
+__device__ __forceinline__ RaggedPos split_pos(const RaggedAttnArgs& a) {
+    int lo = 0, hi = a.items.n - 1;  // the last item that starts at or before this split
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (a.split0[mid] <= blockIdx.x)
+            lo = mid;
+        else
+            hi = mid - 1;
     }
-    return sp;
+    lo = __shfl_sync(0xffffffffu, lo, 0);  // (tells the compiler that the result is warp-uniform)
+    return RaggedPos{a, lo, a.split0[lo], a.split0[lo + 1] - a.split0[lo]};
 }
 
 // phase time stamps of diagnostic builds: slot k of this CTA's row in a.trace
@@ -321,8 +336,9 @@ __device__ __forceinline__ void store_final(const AttnArgs& a, int item, int h, 
 // Merges the per-warp online-softmax states of a CTA (wacc [nw][RS][D] un-normalised,
 // wm / wl [nw][RS]) for heads g0 .. g0+gn-1 of this KV head and stores them: final
 // when the launch has one split, else into the split scratch.
+template <typename Pos>
 __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* wacc, float* wm, float* wl, int nw,
-                                                int RS, int g0, int gn, const SplitPos& sp, int kvh, int ld = 0) {
+                                                int RS, int g0, int gn, const Pos& sp, int kvh, int ld = 0) {
     if (ld == 0) ld = a.kv.D;  // row stride of wacc (the tensor-core kernels pad it against bank conflicts)
     const int D = a.kv.D, G = a.kv.G;
     // one thread per head turns the warps' maxima into weights once (wm <- 2^(m_w - max), wl[g] <- merged l,
@@ -348,10 +364,10 @@ __device__ __forceinline__ void cta_merge_store(const AttnArgs& a, const float* 
         for (int w = 0; w < nw; ++w) o = fmaf(wm[w * RS + g], wacc[(w * RS + g) * ld + d], o);
         const float ms = wx[g], ls = wl[g];
         const int h = kvh * G + g0 + g;
-        if (sp.n == 1) {
-            store_final(a, sp.item, h, d, o, ms, ls);
+        if (sp.n() == 1) {
+            store_final(a, sp.item(), h, d, o, ms, ls);
         } else {
-            float* pp = a.part + (sp.first + (int64_t)h * sp.n + sp.split) * (D + 2);
+            float* pp = a.part + sp.row(h, sp.split()) * (D + 2);
             pp[d] = o;
             if (d == 0) {
                 pp[D] = ms;
@@ -411,13 +427,14 @@ inline size_t split_merge_sub_floats(int G, int D) { return G <= 4 ? (size_t)G *
 // The last CTA of a (token, kv head) to arrive (atomic ticket) merges the
 // per-split states from the scratch buffer and resets the ticket. `wsm` is
 // shared memory for G * n_split weights (the drained ring is reused).
-__device__ __forceinline__ void split_merge_store(const AttnArgs& a, const SplitPos& sp, int kvh, int* s_last, float* wsm) {
-    const int item = sp.item;
-    if (sp.n == 1) {
+template <typename Pos>
+__device__ __forceinline__ void split_merge_store(const AttnArgs& a, const Pos& sp, int kvh, int* s_last, float* wsm) {
+    const int item = sp.item();
+    if (sp.n() == 1) {
         peer_group_done(a);
         return;
     }
-    const int D = a.kv.D, G = a.kv.G, NS = sp.n;
+    const int D = a.kv.D, G = a.kv.G, NS = sp.n();
     // one fence on each side of the ticket, issued by the thread that takes it: the CTA barrier before it orders
     // every thread's stores of this CTA's state ahead of the fence, the barrier after it orders every thread's
     // loads of the other CTAs' states behind it (fences are cumulative)
@@ -431,7 +448,7 @@ __device__ __forceinline__ void split_merge_store(const AttnArgs& a, const Split
     __syncthreads();
     if (!*s_last) return;
     DECODE_STAMP(5);
-    const float* base = a.part + (sp.first + (int64_t)kvh * G * NS) * (D + 2);
+    const float* base = a.part + sp.row(kvh * G, 0) * (D + 2);
     // One warp per head; this CTA runs alone at the end of the launch and a round trip to the states that other
     // SMs just wrote costs about 1.4 us, so everything is arranged for few dependent round trips: (m, l) of all
     // splits in one lane-strided batch of 8-byte loads, the split outputs in batches of 16 or 32 independent
@@ -669,8 +686,8 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_simt_kernel(AttnArgs a) 
     __shared__ int s_last;
 
     const int D = a.kv.D, G = a.kv.G, Hq = a.kv.Hq;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     // the warp index goes through a broadcast so that the compiler knows everything derived from it (key range,
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -687,7 +704,7 @@ __global__ void __launch_bounds__(kSimtWarps * 32) attn_simt_kernel(AttnArgs a) 
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);  // cache row of local position 0

@@ -57,8 +57,9 @@ inline size_t tile_smem_bytes(int nst) {
     return 128 + (body > fold ? body : fold);
 }
 
-template <int FMT, int D>
-__global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
+// Args: AttnArgs, or RaggedAttnArgs for sequences of different lengths
+template <int FMT, int D, typename Args>
+__global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(Args a) {
     using Ge = TileGeom<FMT, D>;
     constexpr int TK = Ge::TK, RS = Ge::RS, NC = Ge::NC, CD = Ge::CD, NSH = Ge::NSH, EPT = Ge::EPT, DT = Ge::DT,
                   KG = Ge::KG, KPG = Ge::KPG, EB = Ge::EB, PIECE = Ge::PIECE;
@@ -66,8 +67,8 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
     __shared__ int s_last;
 
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nst = a.tile_stages;
     DECODE_STAMP(0);
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk;
     const int s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
@@ -321,10 +322,10 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
 #pragma unroll
                 for (int q = 0; q < KG; ++q) o += red[((size_t)q * gh + g) * D + d];
                 const int h = kvh * G + g0 + g;
-                if (sp.n == 1) {
+                if (sp.n() == 1) {
                     store_final(a, item, h, d, o, m_s[g], l_s[g]);
                 } else {
-                    float* pp = a.part + (sp.first + (int64_t)h * sp.n + split) * (D + 2);
+                    float* pp = a.part + sp.row(h, split) * (D + 2);
                     pp[d] = o;
                     if (d == 0) {
                         pp[D] = m_s[g];
@@ -340,10 +341,10 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(AttnArgs a) {
 #pragma unroll
                     for (int e = 0; e < EPT; ++e) {
                         const int d = dt * EPT + e;
-                        if (sp.n == 1) {
+                        if (sp.n() == 1) {
                             store_final(a, item, h, d, acc[g][e], m_s[g], l_s[g]);
                         } else {
-                            float* pp = a.part + (sp.first + (int64_t)h * sp.n + split) * (D + 2);
+                            float* pp = a.part + sp.row(h, split) * (D + 2);
                             pp[d] = acc[g][e];
                             if (d == 0) {
                                 pp[D] = m_s[g];
@@ -402,16 +403,16 @@ inline TilePlan tile_plan(int fmt, int D, int nst, int smem_optin) {
     }
 }
 
-template <int FMT, int D>
-inline int launch_tile_inst(const AttnArgs& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
+template <int FMT, int D, typename Args>
+inline int launch_tile_inst(const Args& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
     static KernelSmemSetup setup;
-    const cudaError_t se = setup.ensure(attn_tile_kernel<FMT, D>, device, smem_optin);
+    const cudaError_t se = setup.ensure(attn_tile_kernel<FMT, D, Args>, device, smem_optin);
     if (se != cudaSuccess) return (int)se;
-    return (int)launch_chained(a.chained, attn_tile_kernel<FMT, D>, grid, kTileThreads, smem, stream, a);
+    return (int)launch_chained(a.chained, attn_tile_kernel<FMT, D, Args>, grid, kTileThreads, smem, stream, a);
 }
 
-template <int FMT>
-inline int launch_tile_fmt(const AttnArgs& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
+template <int FMT, typename Args>
+inline int launch_tile_fmt(const Args& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
     switch (a.kv.D) {
         case 64: return launch_tile_inst<FMT, 64>(a, grid, smem, smem_optin, device, stream);
         case 128: return launch_tile_inst<FMT, 128>(a, grid, smem, smem_optin, device, stream);
@@ -420,7 +421,8 @@ inline int launch_tile_fmt(const AttnArgs& a, dim3 grid, size_t smem, int smem_o
     }
 }
 
-inline int launch_tile_decode(const AttnArgs& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
+template <typename Args>
+inline int launch_tile_decode(const Args& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
     switch (a.kv.fmt) {
         case KV_F32: return launch_tile_fmt<KV_F32>(a, grid, smem, smem_optin, device, stream);
         case KV_BF16: return launch_tile_fmt<KV_BF16>(a, grid, smem, smem_optin, device, stream);

@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(kTurboWarps * 32) attn_turbo_kernel(AttnArgs a
     constexpr int CB = EPL / 4;    // code bytes per lane
     constexpr int SB = EPL / 8;    // sign bytes per lane
     const int G = a.kv.G, Hkv = a.kv.Hkv, kv_dim = a.kv.kv_dim;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int grp = warp * 4 + (lane >> 3), sl = lane & 7;
     const unsigned gmask = 0xffu << (lane & 24);
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kTurboWarps * 32) attn_turbo_kernel(AttnArgs a
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk, s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
     const int k0 = s0 - a.kv.pos_begin, k1 = s1 - a.kv.pos_begin;

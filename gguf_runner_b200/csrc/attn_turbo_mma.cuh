@@ -129,13 +129,14 @@ __device__ __forceinline__ void turbo_mma_expand(const unsigned char* codes, con
     }
 }
 
-__global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs a) {
+template <typename Args>
+__global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(Args a) {
     extern __shared__ __align__(16) unsigned char tsm8[];
     __shared__ int s_last;
     constexpr int D = kTmD, KS = D / 16, NT = D / 8, rowbytes = D * 2;
     const int G = a.kv.G, Hq = a.kv.Hq;
-    const SplitPos sp = split_pos(a);
-    const int split = sp.split, kvh = blockIdx.y, item = sp.item;
+    const auto sp = split_pos(a);
+    const int split = sp.split(), kvh = blockIdx.y, item = sp.item();
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int gq = lane >> 2, tq = lane & 3;
     decode_begin(a);
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     vs = max(vs, a.kv.pos_begin);
     ve = min(ve, a.kv.pos_begin + a.shard_count);
     const int T = max(0, ve - vs);
-    const int chunk = (T + sp.n - 1) / sp.n;
+    const int chunk = (T + sp.n() - 1) / sp.n();
     const int s0 = vs + split * chunk, s1 = min(ve, s0 + chunk);
     const int64_t row0 = a.kv.row(seq, a.layer, a.kv.pos_begin);
     const int k0 = s0 - a.kv.pos_begin, k1 = s1 - a.kv.pos_begin;
@@ -397,11 +398,12 @@ __global__ void __launch_bounds__(kTmWarps * 32) attn_turbo_mma_kernel(AttnArgs 
     split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(tsm8));
 }
 
-inline int launch_turbo_mma(const AttnArgs& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
+template <typename Args>
+inline int launch_turbo_mma(const Args& a, dim3 grid, size_t smem, int smem_optin, int device, cudaStream_t stream) {
     static KernelSmemSetup setup;
-    const cudaError_t se = setup.ensure(attn_turbo_mma_kernel, device, smem_optin);
+    const cudaError_t se = setup.ensure(attn_turbo_mma_kernel<Args>, device, smem_optin);
     if (se != cudaSuccess) return (int)se;
-    return (int)launch_chained(a.chained, attn_turbo_mma_kernel, grid, kTmWarps * 32, smem, stream, a);
+    return (int)launch_chained(a.chained, attn_turbo_mma_kernel<Args>, grid, kTmWarps * 32, smem, stream, a);
 }
 
 }  // namespace ggr

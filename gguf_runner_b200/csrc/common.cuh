@@ -82,10 +82,6 @@ struct Items {
     int mode;  // 0: decode, item b -> (seq b, pos[b]); 1: prefill, item i -> (seq0, base_pos + i)
     int seq0, base_pos, n;
     int pos[kMaxArgItems];
-    // Sequences of different lengths (decode only): item i is split split0[i + 1] - split0[i] ways, and the splits of
-    // all items are numbered one after the other in blockIdx.x. Otherwise every item is split the same way.
-    int ragged;
-    unsigned short split0[kMaxArgItems + 1];
 
     __device__ __forceinline__ void get(int item, int& seq, int& p) const {
         if (mode == 0) {

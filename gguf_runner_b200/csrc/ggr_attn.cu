@@ -548,13 +548,14 @@ struct Lengths {
         for (int i = 0; i < n; ++i) sum += std::max(1, (len[i] + chunk - 1) / chunk);
         return sum;
     }
-    // numbers the splits in `items`
-    void number(int t_max, int splits, Items* items) const {
+    // `a` with the splits numbered over all items
+    RaggedAttnArgs number(const AttnArgs& a, int t_max, int splits) const {
+        RaggedAttnArgs r;
+        static_cast<AttnArgs&>(r) = a;
         const int chunk = (t_max + splits - 1) / splits;
-        items->ragged = 1;
-        items->split0[0] = 0;
-        for (int i = 0; i < n; ++i)
-            items->split0[i + 1] = (unsigned short)(items->split0[i] + std::max(1, (len[i] + chunk - 1) / chunk));
+        r.split0[0] = 0;
+        for (int i = 0; i < n; ++i) r.split0[i + 1] = (unsigned short)(r.split0[i] + std::max(1, (len[i] + chunk - 1) / chunk));
+        return r;
     }
 };
 
@@ -567,7 +568,7 @@ struct Lengths {
 int choose_splits(int64_t base_ctas, int64_t slots, int t_max, int min_keys, int max_splits, double bytes_per_key,
                   double cta_rate, double t_wave = 8e-6, const Lengths* ragged = nullptr) {
     int limit = std::max(1, t_max / std::max(1, min_keys));
-    limit = std::min(limit, ragged ? 511 : 512);  // (511 * kMaxArgItems splits still fit Items::split0)
+    limit = std::min(limit, ragged ? 511 : 512);  // (511 * kMaxArgItems splits still fit split0)
     if (max_splits > 0) limit = std::min(limit, max_splits);
     const double hbm_rate = 6.6e12;
     int best = 1;
@@ -774,8 +775,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         }
         n_split = std::min(n_split, limit);
         ragged = ragged && tc && n_split > 1;
-        if (ragged) lengths.number(t_max, n_split, &a.items);
-        const int total = ragged ? a.items.split0[items.n] : items.n * n_split;
+        const int total = ragged ? lengths.total(t_max, n_split) : items.n * n_split;
         const dim3 grid = ragged ? dim3(total, c->kv.Hkv, 1) : dim3(n_split, c->kv.Hkv, items.n);
         a.n_split = n_split;
         c->last_splits = n_split;
@@ -789,7 +789,8 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             const size_t smem = turbo_mma_smem_bytes(c->G, n_split);
             a.stage_bytes = (int)turbo_mma_prep_offset(c->G, n_split);
             LaunchTimer t(c, 0);
-            e = launch_turbo_mma(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
+            e = ragged ? launch_turbo_mma(lengths.number(a, t_max, n_split), grid, smem, c->smem_optin, c->cfg.device, c->stream)
+                       : launch_turbo_mma(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         } else {
             const size_t smem = turbo_attn_smem_floats(c->D, c->G, turbo_heads_per_pass(c->G, c->D), n_split) * sizeof(float);
             if (smem + 1024 > (size_t)c->smem_optin)
@@ -809,7 +810,6 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     if (ragged) {
         const size_t fit = c->part_cap / ((size_t)c->kv.Hq * (c->D + 2));  // splits of all items the reservation holds
         while (c->reserved_batch > 0 && n_split > 1 && (size_t)lengths.total(t_max, n_split) > fit) --n_split;
-        ragged = n_split > 1;
     } else {
         // with a reservation in place the split count never outgrows the reserved scratch (as long as that
         // holds two splits): the decode loop then neither allocates nor synchronises for memory
@@ -850,8 +850,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
 
     a.n_split = n_split;
     c->last_splits = n_split;
-    if (ragged) lengths.number(t_max, n_split, &a.items);
-    const int total_splits = ragged ? a.items.split0[items.n] : items.n * n_split;
+    const int total_splits = ragged ? lengths.total(t_max, n_split) : items.n * n_split;
     // the split merge stages one weight per (head, split) in shared memory
     const size_t merge_smem = split_merge_smem_bytes(c, n_split);
     smem = std::max(smem, merge_smem);
@@ -887,8 +886,10 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         int rc;
         {
             LaunchTimer t(c, 0);
-            rc = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, dp.warps, grid, smem, c->smem_optin, c->cfg.device, c->stream)
-                     : launch_mma_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
+            rc = ragged ? launch_mma_tma_decode(c->tmK16, c->tmV16, lengths.number(a, t_max, n_split), grid, smem, c->smem_optin,
+                                                c->cfg.device, c->stream)
+                 : tma  ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, grid, smem, c->smem_optin, c->cfg.device, c->stream)
+                        : launch_mma_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (rc != 0) return fail(c, GGR_ERR_CUDA, std::string("mma decode launch: ") + cudaGetErrorString((cudaError_t)rc));
         c->launches++;
@@ -898,7 +899,8 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
         int rc;
         {
             LaunchTimer t(c, 0);
-            rc = launch_tile_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
+            rc = ragged ? launch_tile_decode(lengths.number(a, t_max, n_split), grid, smem, c->smem_optin, c->cfg.device, c->stream)
+                        : launch_tile_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (rc != 0) return fail(c, GGR_ERR_CUDA, std::string("tile decode launch: ") + cudaGetErrorString((cudaError_t)rc));
         c->launches++;
@@ -2201,7 +2203,7 @@ extern "C" int ggr_attn_attention_tokens_static(ggr_attn_ctx* c, int32_t layer, 
         int e;
         {
             LaunchTimer t(c, 0);
-            e = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, dp.warps, grid, smem, c->smem_optin, c->cfg.device, c->stream)
+            e = tma ? launch_mma_tma_decode(c->tmK16, c->tmV16, a, grid, smem, c->smem_optin, c->cfg.device, c->stream)
                     : launch_mma_decode(a, grid, smem, c->smem_optin, c->cfg.device, c->stream);
         }
         if (e != 0) return fail(c, GGR_ERR_CUDA, std::string("mma decode launch: ") + cudaGetErrorString((cudaError_t)e));
