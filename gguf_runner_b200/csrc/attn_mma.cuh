@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     // ring addresses, TMA coordinates) is warp-uniform
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int gq = lane >> 2, tq = lane & 3;
-    const bool ahead = decode_ahead(a, item, kvh);
+    const bool ahead = decode_ahead(a);
     if (!ahead) decode_begin(a);
 
     int seq, pos;
@@ -566,6 +566,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attn_mma_tma_decode_kernel(cons
     decode_tail(a);
     split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem_al));
     DECODE_STAMP(4);
+    decode_leave(a);
 }
 
 template <int D, int W>

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(Args a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nst = a.tile_stages;
     DECODE_STAMP(0);
-    const bool ahead = decode_ahead(a, item, kvh);
+    const bool ahead = decode_ahead(a);
     if (!ahead) decode_begin(a);
 
     int seq, pos;
@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kTileThreads) attn_tile_kernel(Args a) {
     decode_tail(a);
     split_merge_store(a, sp, kvh, &s_last, reinterpret_cast<float*>(smem));
     DECODE_STAMP(4);
+    decode_leave(a);
 }
 
 inline bool tile_decode_supported(int fmt, int D) {

@@ -99,7 +99,8 @@ struct ggr_attn_ctx {
     std::vector<void*> retired;    // scratch that was outgrown after that, kept for the graphs
     bool host_call = false;  // the decode call in progress has host pointers: copies stand between its kernels
     int tail_layer = -1;     // layer that the last chained decode launch appended to; -1: none, or an exchange's
-    int* d_sched = nullptr;  // work counters of the persistent prefill kernel (rewound by the kernel itself)
+    // work counters of the persistent prefill kernel (rewound by the kernel itself), and AttnArgs::running
+    int* d_sched = nullptr;
     // per-layer pre-attention fixups (device arrays, null = absent) and their f32 scratch rows
     struct LayerFixups {
         float *q_bias = nullptr, *k_bias = nullptr, *v_bias = nullptr, *q_norm = nullptr, *k_norm = nullptr;
@@ -870,8 +871,10 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     if (a.chained && a.fused.enabled && !px) {
         if (front_ours)
             a.ahead = kAheadKnown;
-        else if (n_split > 1 && c->tail_layer >= 0 && c->tail_layer != layer)
-            a.ahead = kAheadTicket;
+        else if (c->tail_layer >= 0 && c->tail_layer != layer)
+            a.ahead = kAheadRunning;
+        a.running = reinterpret_cast<unsigned*>(c->d_sched) + 2;
+        a.first_wave = c->sm_count * dp.ctas_per_sm;
     }
     const dim3 grid = ragged ? dim3(total_splits, c->kv.Hkv, 1) : dim3(n_split, c->kv.Hkv, items.n);
 #ifdef GGR_TC_TRACE
@@ -1572,11 +1575,11 @@ int ggr_attn_create(const ggr_attn_config* cfg, ggr_attn_ctx** out) {
         return cleanup(GGR_ERR_ALLOC, "unable to allocate the error word");
     }
     *c->h_err = 0;
-    if (cudaMalloc((void**)&c->d_sched, 2 * sizeof(int)) != cudaSuccess) {
+    if (cudaMalloc((void**)&c->d_sched, 3 * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         return cleanup(GGR_ERR_ALLOC, "unable to allocate the prefill work counters");
     }
-    cudaMemsetAsync(c->d_sched, 0, 2 * sizeof(int), c->stream);
+    cudaMemsetAsync(c->d_sched, 0, 3 * sizeof(int), c->stream);
     if (prefill_tc_shape_ok(kv.fmt, c->D) && rows < ((size_t)1 << 31)) {
         c->have_tmaps = make_tmap_bf16(&c->tmK, kv.k, (uint64_t)c->kv_dim, (uint64_t)rows) &&
                         make_tmap_bf16(&c->tmV, kv.v, (uint64_t)c->kv_dim, (uint64_t)rows);
