@@ -98,6 +98,13 @@ struct ggr_attn_ctx {
     bool captured = false;         // launches of this context have been captured into a graph
     std::vector<void*> retired;    // scratch that was outgrown after that, kept for the graphs
     bool host_call = false;  // the decode call in progress has host pointers: copies stand between its kernels
+    struct SplitMemo {
+        int n_items = 0, t_max = 0, max_splits = 0;
+        int family = 0;  // of kernels: 1 tensor core, 2 CTA tile, 0 per-warp rings
+        int splits = 0, stages = 0;  // splits 0: empty
+        std::vector<int> lens;       // of a ragged batch
+    } split_memo[4];
+    int split_memo_next = 0;
     int tail_layer = -1;     // layer that the last chained decode launch appended to; -1: none, or an exchange's
     // work counters of the persistent prefill kernel (rewound by the kernel itself), and AttnArgs::running
     int* d_sched = nullptr;
@@ -541,6 +548,21 @@ int launch_simt(ggr_attn_ctx* c, const AttnArgs& a, dim3 grid, const SimtPlan& p
 // Visible lengths of the sequences of a decode call.
 struct Lengths {
     int n = 0, len[kMaxArgItems];
+    // step over the candidates 1 .. limit, so that at most kSearch lengths are divided
+    static constexpr int kSearch = 4096;
+    int step(int limit) const { return std::max(1, (limit * n + kSearch - 1) / kSearch); }
+    // the largest count up to `splits` whose total is at most `fit`, or 1 (totals grow with the count)
+    int largest(int t_max, int splits, size_t fit) const {
+        int lo = 1, hi = splits;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if ((size_t)total(t_max, mid) <= fit)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        return lo;
+    }
     bool ragged() const { return n > 1 && *std::min_element(len, len + n) != *std::max_element(len, len + n); }
     // splits of all items when the longest (t_max keys) is split `splits` ways and the others into pieces of that size
     int total(int t_max, int splits) const {
@@ -574,7 +596,7 @@ int choose_splits(int64_t base_ctas, int64_t slots, int t_max, int min_keys, int
     const double hbm_rate = 6.6e12;
     int best = 1;
     double best_cost = -1.0;
-    const int step = ragged ? std::max(1, limit * ragged->n / 4096) : 1;  // (bounds the host time of a call)
+    const int step = ragged ? ragged->step(limit) : 1;
     for (int n = 1; n <= limit; n += step) {
         const int64_t ctas = base_ctas * (ragged ? ragged->total(t_max, n) : n);
         const int64_t full = ctas / slots, rem = ctas % slots;
@@ -660,7 +682,7 @@ DecodePlan decode_plan(const ggr_attn_ctx* c, bool allow_mma) {
 
 // Split-KV factor of a launch. The CTA-tile kernel streams with one ring stage when every CTA gets a single tile
 // and with two otherwise, which changes its occupancy and so the split count: settle both here.
-int plan_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits, const Lengths* ragged = nullptr) {
+int search_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits, const Lengths* ragged) {
     auto pick = [&]() {
         return choose_splits((int64_t)c->kv.Hkv * (ragged ? 1 : n_items), (int64_t)c->sm_count * d.ctas_per_sm, t_max, d.min_keys,
                              max_splits, 2.0 * c->D * c->kv.elem_bytes, d.cta_rate, d.tile ? 3e-6 : 8e-6, ragged);
@@ -671,6 +693,26 @@ int plan_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, in
         n = pick();
     }
     return n;
+}
+
+// The layers of a token step ask for the same plans one after the other; the search takes the host 0.8 us for one sequence
+// of 1500 keys and 18 us for 128 of up to 8000, so its last results are kept (four: layers with and without a window, ragged
+// batches planned both ways). (48 sequences, 32/4 heads, bf16: 16.4 -> 11.3 us per decode call until it returns.)
+int plan_splits(ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits, const Lengths* ragged = nullptr) {
+    const int family = d.mma + 2 * d.tile;
+    for (const auto& m : c->split_memo) {
+        if (m.splits == 0 || m.n_items != n_items || m.t_max != t_max || m.max_splits != max_splits || m.family != family ||
+            m.lens.size() != (ragged ? (size_t)ragged->n : 0) || (ragged && !std::equal(m.lens.begin(), m.lens.end(), ragged->len)))
+            continue;
+        if (d.tile) use_tile_plan(c, d, m.stages);
+        return m.splits;
+    }
+    const int splits = search_splits(c, d, n_items, t_max, max_splits, ragged);
+    auto& m = c->split_memo[c->split_memo_next];
+    c->split_memo_next = (c->split_memo_next + 1) % 4;
+    m = {n_items, t_max, max_splits, family, splits, d.tp.nst, {}};
+    if (ragged) m.lens.assign(ragged->len, ragged->len + ragged->n);
+    return splits;
 }
 
 // Partial-state floats and tickets (zero between launches) of a split launch; nothing grows within a reservation.
@@ -764,7 +806,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
             // rounds of its eight warps plus a prologue and merge of about four rounds, and the launch as many of these
             // as it has waves (one CTA per SM). 7777 keys, 4 KV heads: 30 splits of three rounds -> 37 of two.
             int64_t best = -1;
-            for (int n = 1; n <= limit; ++n) {
+            for (int n = 1; n <= limit; n += ragged ? lengths.step(limit) : 1) {
                 const int64_t ctas = ragged ? (int64_t)c->kv.Hkv * lengths.total(t_max, n) : base_ctas * n;
                 const int64_t waves = (ctas + c->sm_count - 1) / c->sm_count;
                 const int64_t cost = waves * (((t_max + n - 1) / n + per_cta_keys - 1) / per_cta_keys + 4);
@@ -810,7 +852,7 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     int n_split = plan_splits(c, dp, items.n, t_max, c->cfg.max_splits, ragged ? &lengths : nullptr);
     if (ragged) {
         const size_t fit = c->part_cap / ((size_t)c->kv.Hq * (c->D + 2));  // splits of all items the reservation holds
-        while (c->reserved_batch > 0 && n_split > 1 && (size_t)lengths.total(t_max, n_split) > fit) --n_split;
+        if (c->reserved_batch > 0) n_split = lengths.largest(t_max, n_split, fit);
     } else {
         // with a reservation in place the split count never outgrows the reserved scratch (as long as that
         // holds two splits): the decode loop then neither allocates nor synchronises for memory
