@@ -730,6 +730,32 @@ int split_scratch(ggr_attn_ctx* c, bool prefill, size_t floats, size_t tickets, 
     return GGR_OK;
 }
 
+// Whether a batch of different lengths goes to the ragged launch (`nr` splits of the longest), or like one of equal lengths
+// to `u` (`nu` splits of every sequence). Measured on a B200, us per layer, ragged / uniform, by mean over longest length,
+// lengths in random order:
+//   TMA-fed tensor-core kernel. More CTAs than SMs: the ragged form, which balances its waves (24 x 3000 keys, 40/8 heads, 0.9:
+//   50 / 59, 0.43: 33 / 41; 32 x 1000, 32/8, 0.6: 23 / 25; 48 x 8000, 32/4, 0.9: 120 / 121, 0.29: 53 / 60; the other way round
+//   only for 48 x 8000, 32/8, 0.9: 221 / 210). One CTA per SM: the ragged form moves 6.2 TB/s at best and costs some 7 us in
+//   pieces, so it pays where the longest piece of the uniform launch, alone on its SM, takes longer than that (8 x 32768,
+//   32/4, 0.999: 87 / 83, 0.6: 58 / 65, 0.31: 38 / 56; 16 x 4000, 32/8, 0.75: 40 / 38, 0.43: 27 / 33; 16 x 1000, 40/8, 0.7:
+//   19 / 16, 0.3: 15 / 14; 2 x 6000, 32/4, 0.6: 16 / 14).
+//   CTA-tile kernel (bound by arithmetic). The ragged form, except where it puts a third CTA on some SMs (q8, 4 x 1500, 32/8,
+//   0.75: 24 / 21, 0.6: 23 / 20, but 0.47: 15 / 20; q8 blocks, 8 x 8000, 32/4, 0.6: 78 / 66), and for nearly equal lengths of
+//   other than bf16 caches (0.9: f32, 8 x 2000, 16/8: 74 / 67, q8, 48 x 4000, 32/8: 366 / 340; bf16, 16 x 4000, 16/8: 110 / 116).
+//   f32, 8 x 2000, 16/8, 0.44: 38 / 67; q8, 16 x 4000, 32/8, 0.3: 54 / 73.
+bool ragged_pays(const ggr_attn_ctx* c, const DecodePlan& u, int nu, int nr, int t_max, const Lengths& lengths) {
+    double keys = 0.0;
+    for (int i = 0; i < lengths.n; ++i) keys += lengths.len[i];
+    if (u.tma) {
+        if (c->kv.Hkv * lengths.n * nu > c->sm_count) return true;
+        const double bytes_per_key = 2.0 * c->D * c->kv.elem_bytes;
+        return (t_max + nu - 1) / nu * bytes_per_key / u.cta_rate > keys * c->kv.Hkv * bytes_per_key / 6.2e12 + 7e-6;
+    }
+    const int ctas = c->kv.Hkv * lengths.total(t_max, nr);
+    if (ctas > 2 * c->sm_count && ctas <= 5 * c->sm_count / 2) return false;
+    return keys < 0.85 * lengths.n * t_max || c->kv.fmt == KV_BF16;
+}
+
 // Output gate of a call (src/engine/runtime/inference.rs:3509-3519); p == nullptr = none.
 struct GateSpec {
     const void* p;
@@ -770,7 +796,8 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     }
 
     // Decode of sequences of different lengths: pieces of one size instead of one number of pieces, so that no CTA has
-    // more to do than another. (16 sequences of 200 to 6000 keys, 40/8 heads of 128, bf16: 45 -> 31 us per layer.)
+    // more to do than another, where that pays (ragged_pays). (16 sequences of 200 to 6000 keys, 40/8 heads of 128, bf16: 45
+    // -> 31 us per layer.)
     Lengths lengths;
     if (items.mode == 0 && items.n > 1) {
         for (int i = 0; i < items.n; ++i) {
@@ -848,8 +875,17 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
 
     DecodePlan dp = decode_plan(c, allow_mma);
     ragged = ragged && (dp.tma || dp.tile);
-    if (ragged && dp.tma) use_tma_plan(c, dp, kTmaWarpsRagged);
-    int n_split = plan_splits(c, dp, items.n, t_max, c->cfg.max_splits, ragged ? &lengths : nullptr);
+    DecodePlan rp = dp;
+    int n_split = plan_splits(c, dp, items.n, t_max, c->cfg.max_splits);
+    if (ragged) {
+        if (rp.tma) use_tma_plan(c, rp, kTmaWarpsRagged);
+        const int nr = plan_splits(c, rp, items.n, t_max, c->cfg.max_splits, &lengths);
+        ragged = ragged_pays(c, dp, n_split, nr, t_max, lengths);
+        if (ragged) {
+            dp = rp;
+            n_split = nr;
+        }
+    }
     if (ragged) {
         const size_t fit = c->part_cap / ((size_t)c->kv.Hq * (c->D + 2));  // splits of all items the reservation holds
         if (c->reserved_batch > 0) n_split = lengths.largest(t_max, n_split, fit);
