@@ -320,8 +320,12 @@ inline MmaPlan mma_tma_plan(int D, int warps, int smem_optin) {
     p.ctas_per_sm = (int)((size_t)(smem_optin + 1024) / (p.smem + 4096));
     if (p.ctas_per_sm < 1) p.ctas_per_sm = 1;
     if (p.ctas_per_sm > 4) p.ctas_per_sm = 4;
-    // eight warps: down to one tile per warp (2000 keys, 8 KV heads: 7 splits of three rounds -> 16 of one)
-    p.min_keys = warps == kTmaWarps ? warps * kTmaTK - 8 : warps * kTmaTK * 2;
+    // Keys of the smallest split: one tile per warp for eight warps, two for four. Bound by the rounds of its warps, so the
+    // last split may be smaller, and a split never has a few keys more (plan_splits rounds up). us per layer from a graph, 32/8 | 32/4
+    // heads, two tiles per warp -> one: 700 keys 11.2 -> 10.7 | 12.2 -> 11.6, 1000: 12.1 -> 10.6 | 12.8 -> 11.9, 1300: 12.2
+    // -> 10.8 | 13.0 -> 12.0, 2000: 12.6 -> 12.0 | 13.2 -> 12.3, 3000: 13.4 -> 13.6 | 13.3 -> 12.9, 4000: 13.9 -> 14.0 | 14.2
+    // -> 13.6; up to 450 keys unsplit either way.
+    p.min_keys = warps == kTmaWarps ? warps * kTmaTK : warps * kTmaTK * 2;
     return p;
 }
 

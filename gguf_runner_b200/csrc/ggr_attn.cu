@@ -588,9 +588,9 @@ struct Lengths {
 // costs a little per split. The constants are measured on B200 (TMA-fed decode kernel: ~65 GB/s per
 // CTA alone, ~6.6 TB/s for the whole GPU, ~8 us per wave). Picks the n with the smallest modelled time. For a ragged
 // batch n is the split count of the longest sequence, and base_ctas counts the CTAs of one split of one sequence.
-int choose_splits(int64_t base_ctas, int64_t slots, int t_max, int min_keys, int max_splits, double bytes_per_key,
+int choose_splits(int64_t base_ctas, int64_t slots, int t_max, int most, int max_splits, double bytes_per_key,
                   double cta_rate, double t_wave = 8e-6, const Lengths* ragged = nullptr) {
-    int limit = std::max(1, t_max / std::max(1, min_keys));
+    int limit = std::max(1, most);
     limit = std::min(limit, ragged ? 511 : 512);  // (511 * kMaxArgItems splits still fit split0)
     if (max_splits > 0) limit = std::min(limit, max_splits);
     const double hbm_rate = 6.6e12;
@@ -683,8 +683,10 @@ DecodePlan decode_plan(const ggr_attn_ctx* c, bool allow_mma) {
 // Split-KV factor of a launch. The CTA-tile kernel streams with one ring stage when every CTA gets a single tile
 // and with two otherwise, which changes its occupancy and so the split count: settle both here.
 int search_splits(const ggr_attn_ctx* c, DecodePlan& d, int n_items, int t_max, int max_splits, const Lengths* ragged) {
+    // splits of the smallest size that a sequence of t_max keys has
+    auto most = [&]() { return (t_max + (d.tma && d.warps == kTmaWarps ? d.min_keys - 1 : 0)) / std::max(1, d.min_keys); };
     auto pick = [&]() {
-        return choose_splits((int64_t)c->kv.Hkv * (ragged ? 1 : n_items), (int64_t)c->sm_count * d.ctas_per_sm, t_max, d.min_keys,
+        return choose_splits((int64_t)c->kv.Hkv * (ragged ? 1 : n_items), (int64_t)c->sm_count * d.ctas_per_sm, t_max, most(),
                              max_splits, 2.0 * c->D * c->kv.elem_bytes, d.cta_rate, d.tile ? 3e-6 : 8e-6, ragged);
     };
     int n = pick();
