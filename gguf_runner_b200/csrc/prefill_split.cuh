@@ -5,7 +5,8 @@
 // centroids, which are alpha * {-6128, -1837, 1837, 6128} to 2e-8 (the f32 constants themselves are only given to
 // 3e-8). All of them are exact in f16. The other operand of each product (q, or the softmax weight times the value
 // scale) is an f32 number x, scaled by a power of two into f16's range and split as x = hi + lo with two f16 of 11
-// significant bits each: what is left out is below 2^-24 |x|, f32's own rounding. So
+// significant bits each: what is left out is at most 2^-23 |x|, one bit more than f32's rounding, or 2^-38 of the largest
+// element that shares the power of two (lo of an element 2^-15 below that is subnormal). So
 //   q . code = hi . code + lo . code     and     P V = P_hi V + P_lo V
 // are two f16 MMAs with f32 accumulation; the scales are applied in f32, and the sums over the keys of one tile are
 // added to the running output by f32 additions, so no accumulation in the tensor core is longer than 64 keys.
@@ -19,9 +20,13 @@
 //          the partial scores change hands through shared memory, and each keeps one of the two output accumulators.
 // Where the row tiles do not fill the GPU, the keys are split over CTAs and the last one of a tile merges.
 //
-// Bound: issue rate of mma.sync (256 MMAs of 16 x 8 x 16 per warp and tile) and the softmax between them. Measured on a
-// B200, per layer, against the f32 CUDA-core kernels (attn_simt_kernel, attn_turbo_kernel), rope and append included:
-// 32/8 heads of 128, 1000 rows, q8: 1464 -> 106 us; 16/8 heads, 512 rows behind 700, TurboQuant: 1200 -> 154 us.
+// The other places that are not f32 FMAs: the centroids' common factor (2e-8) and the sums of 16 products, which the tensor
+// core rounds in its own way. Outputs against 64-bit attention over the same cache: q8 1000 rows, 3.2e-5 (the angles of RoPE),
+// as the f32 CUDA-core kernel; the two kernels differ by 2.3e-7 there and by 5.6e-7 for 512 TurboQuant rows.
+//
+// Bound: latency of a chain per warp (expand, barrier, Q K^T, softmax, split, P V) at eight warps per SM, 255 registers each.
+// Measured on a B200, per layer, against the f32 CUDA-core kernels (attn_simt_kernel, attn_turbo_kernel), rope and append
+// included: 32/8 heads of 128, 1000 rows, q8: 1464 -> 106 us; 16/8 heads, 512 rows behind 700, TurboQuant: 1200 -> 130 us.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -57,7 +62,7 @@ __device__ __forceinline__ void mma_f16_16816(float* c, const uint32_t* a, uint3
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// (x, y) -> f16 pairs hi and lo with hi + lo = (x, y) to 2^-24
+// (x, y) -> f16 pairs hi and lo with hi + lo = (x, y) to 2^-23, for x and y in f16's normal range
 __device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x, y);
     const float2 f = __half22float2(h);

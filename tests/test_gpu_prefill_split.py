@@ -2,7 +2,8 @@
 (prefill_impl = SIMT) on the same rows, at the edges of its 64-row and 64-key tiles.
 
 Tolerance: both kernels round every product and sum to f32. A score of head_dim N(0, 1) products carries an error of
-about sqrt(128) * 2^-24 * |q| |k| / sqrt(128) = 2^-24 * 11.3 * 11.3 = 7.6e-6, which is the relative error of its softmax
+about sqrt(128) * 2^-24 * |q| |k| / sqrt(128) = 2^-24 * 11.3 * 11.3 = 7.6e-6 (the two f16 parts of an operand leave out up to
+2^-23 of it, but independently per element: they add less than half of that), which is the relative error of its softmax
 weight; outputs are weighted means of values up to ~4.5, so two such evaluations differ by less than 7e-5.
 """
 import numpy as np
