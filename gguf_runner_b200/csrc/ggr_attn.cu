@@ -812,8 +812,8 @@ int launch_attention(ggr_attn_ctx* c, int layer, const Items& items, int t_max, 
     bool ragged = lengths.ragged();
 
     if (c->kv.fmt == KV_TURBO) {
-        // TurboQuant cache: rope + quantising append as separate launches, then the CUDA-core attention kernel.
-        // Splits fill the GPU about four CTAs deep (the kernel is bound by arithmetic, not by HBM).
+        // TurboQuant cache: rotation and quantising append in launches of their own (one, turbo_prep_kernel, for heads of
+        // 128 rotated as a whole), then attention.
         if (raw) {
             int rc = launch_rope_append(c, layer, items, RF_ROTATE | RF_WRITE_Q | RF_APPEND, 0, raw->q, raw->k, raw->v,
                                         const_cast<float*>(q_dev), nullptr, nullptr);
